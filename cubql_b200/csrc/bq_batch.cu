@@ -27,16 +27,18 @@
 // cloud).  Clouds with empty boxes are not supported in batches.
 //
 // Batched kNN: queries are also stored cloud by cloud; they are sorted by
-// (cloud, 30-bit Morton code in the cloud's root box) and answered by a
+// (cloud, 30-bit Hilbert position in the cloud's root box).  Under the
+// lowest-id rule each warp makes one search for its 32 queries
+// (bq_group.cuh); the reference's rule, k > 32 and unsorted queries take a
 // persistent work-stealing kernel (one CTA per SM slot; warps grab chunks
 // of `queriesPerWarp` queries from a global counter until the batch is
-// exhausted), which keeps all SMs busy despite very uneven clouds.
+// exhausted).
 #include <algorithm>
 #include <climits>
 #include <cfloat>
 
 #include "bq_agglom.cuh"
-#include "bq_traverse.cuh"
+#include "bq_group.cuh"
 
 namespace bq {
 int query_config(const bq_query_config *q, bq_query_config &out);
@@ -309,16 +311,8 @@ __global__ void k_seg_query_keys(const bq_bvh3f *__restrict__ bvhs, const float 
   const uint32_t s = seg_of(qoff, numSegs, t);
   uint32_t code = 0;
   const bq_bvh3f d = bvhs[s];
-  if (d.numNodes) {
-    const Node root = ldg_node((const Node *)d.nodes);
-    const float ext = fmaxf(fmaxf(root.a.w - root.a.x, root.b.x - root.a.y), root.b.y - root.a.z);
-    const float sc = 1024.0f / fmaxf(ext, 1e-20f);
-    const float *q = queries + 3ull * t;
-    const uint32_t cx = min(__float2uint_rz((q[0] - root.a.x) * sc), 1023u);
-    const uint32_t cy = min(__float2uint_rz((q[1] - root.a.y) * sc), 1023u);
-    const uint32_t cz = min(__float2uint_rz((q[2] - root.a.z) * sc), 1023u);
-    code = spread10(cx) | (spread10(cy) << 1) | (spread10(cz) << 2);
-  }
+  if (d.numNodes)
+    code = query_order_key((const float *)d.nodes, queries + 3ull * t);
   keys[t] = ((uint64_t)s << 32) | code;
   idx[t] = t;
 }
@@ -342,6 +336,76 @@ struct BKnnLeaf {
     return fminf(maxSqr, list.worst());
   }
 };
+
+template <int K, int TIE>
+__device__ __forceinline__ void write_knn(const KnnList<K, TIE> &list, uint32_t qi, int k, int32_t *outIds,
+                                          float *outD, int32_t *numFound)
+{
+  int found = 0;
+  int32_t *oi = outIds + (size_t)qi * k;
+  float *od = outD + (size_t)qi * k;
+#pragma unroll
+  for (int j = 0; j < K; j++) {
+    if (j >= K - k) {
+      const bool real = list.real(j);
+      oi[j - (K - k)] = real ? list.id(j) : -1;
+      od[j - (K - k)] = real ? list.dist(j) : INFINITY;
+      found += real ? 1 : 0;
+    }
+  }
+  if (numFound) numFound[qi] = found;
+}
+
+// one search for a warp's 32 queries (bq_group.cuh), or one for each cloud
+// that they belong to; queries that cannot share it are answered one thread
+// each
+template <int K, int STACK>
+__global__ void __launch_bounds__(128, GroupShape<K>::BLOCKS)
+    k_seg_knn_warp(const bq_bvh3f *__restrict__ bvhs, const uint32_t *__restrict__ poff,
+                   const float *__restrict__ points, const float *__restrict__ queries,
+                   const uint32_t *__restrict__ qoff, const uint64_t *__restrict__ sortedKeys,
+                   const uint32_t *__restrict__ order, uint32_t nq, int k, float maxSqr, int32_t *__restrict__ outIds,
+                   float *__restrict__ outD, int32_t *__restrict__ numFound, uint32_t *__restrict__ ovfList,
+                   uint32_t *ovfCount)
+{
+  griddep_wait();
+  __shared__ GroupShared<K> sh[4];
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool alive = t < nq;
+  const uint32_t tt = min(t, nq - 1);
+  const uint32_t qi = __ldg(order + tt);
+  const uint32_t s = (uint32_t)(__ldg(sortedKeys + tt) >> 32);
+  const float *q = queries + 3ull * qi;
+  BKnnLeaf<K, TIE_LOWEST> leaf;
+  leaf.qx = __ldg(q); leaf.qy = __ldg(q + 1); leaf.qz = __ldg(q + 2);
+  leaf.maxSqr = maxSqr;
+  leaf.list.init(k);
+  uint32_t todo = __ballot_sync(0xffffffffu, alive);
+  while (todo) {
+    const uint32_t s0 = __shfl_sync(0xffffffffu, s, __ffs(todo) - 1);
+    const bool mine = alive && s == s0;
+    todo &= ~__ballot_sync(0xffffffffu, mine);
+    const bq_bvh3f d = bvhs[s0];
+    const Node *nodes = (const Node *)d.nodes;
+    leaf.primIDs = d.primIDs;
+    leaf.points = points + 3ull * __ldg(poff + s0);
+    bool in = false, done = false;
+    if (d.numNodes && group_pays(__ldg(qoff + s0 + 1) - __ldg(qoff + s0), d.numPrims)) {
+      in = mine && group_can_search(nodes, leaf.qx, leaf.qy, leaf.qz);
+      done = group_search<K>(nodes, d.primIDs, leaf.points, in, leaf.qx, leaf.qy, leaf.qz, maxSqr, leaf.list,
+                             sh[threadIdx.x >> 5]);
+    }
+    if (mine && d.numNodes && !(done && in)) {
+      const float seed = in ? fminf(maxSqr, leaf.list.worst()) : maxSqr;
+      leaf.list.init(k);
+      LocalStack<STACK> st;
+      if (!traverse<TIE_LOWEST>(nodes, leaf.qx, leaf.qy, leaf.qz, seed, st, leaf)) ovfList[atomicAdd(ovfCount, 1u)] = t;
+    }
+    __syncwarp();
+  }
+  // (a query on the overflow list is written again by the deep-stack kernel)
+  if (alive) write_knn(leaf.list, qi, k, outIds, outD, numFound);
+}
 
 template <int K, int TIE, int STACK>
 __global__ void __launch_bounds__(128) k_seg_knn(const bq_bvh3f *__restrict__ bvhs,
@@ -385,17 +449,7 @@ __global__ void __launch_bounds__(128) k_seg_knn(const bq_bvh3f *__restrict__ bv
         ovfList[atomicAdd(ovfCount, 1u)] = t;
         continue;
       }
-      int found = 0;
-#pragma unroll
-      for (int j = 0; j < K; j++) {
-        if (j >= K - k) {
-          const bool real = leaf.list.real(j);
-          oi[j - (K - k)] = real ? leaf.list.id(j) : -1;
-          od[j - (K - k)] = real ? leaf.list.dist(j) : INFINITY;
-          found += real ? 1 : 0;
-        }
-      }
-      if (numFound) numFound[qi] = found;
+      write_knn(leaf.list, qi, k, outIds, outD, numFound);
     }
   }
 }
@@ -448,14 +502,18 @@ constexpr int DEEP_STACK = 1024;
 
 template <int K, int TIE, int STACK>
 int launch_seg_knn(const bq_bvh3f *bvhs, const uint32_t *poff, const float *points, const float *queries,
-                   const uint64_t *skeys, const uint32_t *order, uint32_t nq, int k, float maxSqr, int block,
-                   int chunk, uint32_t *workCtr, int32_t *ids, float *d, int32_t *nf, uint32_t *ovfList,
+                   const uint32_t *qoff, const uint64_t *skeys, const uint32_t *order, uint32_t nq, int k, float maxSqr,
+                   int block, int chunk, uint32_t *workCtr, int32_t *ids, float *d, int32_t *nf, uint32_t *ovfList,
                    uint32_t *ovfCount, StackEntry *deep, uint32_t *err, cudaStream_t s)
 {
-  int perSm = 0;
-  BQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_seg_knn<K, TIE, STACK>, block, 0));
-  const int grid = std::max(1, std::min(num_sms() * std::max(perSm, 1), div_up(nq, block)));
-  {
+  if (TIE == TIE_LOWEST && K <= 32 && order) {
+    ProfScope ps("batch.knn", s);
+    launch_pdl(k_seg_knn_warp<K <= 32 ? K : 32, STACK>, dim3(div_up(nq, block)), dim3(block), 0, s, bvhs, poff, points,
+               queries, qoff, skeys, order, nq, k, maxSqr, ids, d, nf, ovfList, ovfCount);
+  } else {
+    int perSm = 0;
+    BQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_seg_knn<K, TIE, STACK>, block, 0));
+    const int grid = std::max(1, std::min(num_sms() * std::max(perSm, 1), div_up(nq, block)));
     ProfScope ps("batch.knn", s);
     launch_pdl(k_seg_knn<K, TIE, STACK>, dim3(grid), dim3(block), 0, s, bvhs, poff, points, queries, skeys, order, nq,
                k, maxSqr, chunk, workCtr, ids, d, nf, ovfList, ovfCount);
@@ -469,18 +527,18 @@ int launch_seg_knn(const bq_bvh3f *bvhs, const uint32_t *poff, const float *poin
 
 template <int K, int TIE>
 int stack_dispatch(int stack, const bq_bvh3f *bvhs, const uint32_t *poff, const float *points, const float *queries,
-                   const uint64_t *skeys, const uint32_t *order, uint32_t nq, int k, float maxSqr, int block,
-                   int chunk, uint32_t *workCtr, int32_t *ids, float *d, int32_t *nf, uint32_t *ovfList,
+                   const uint32_t *qoff, const uint64_t *skeys, const uint32_t *order, uint32_t nq, int k, float maxSqr,
+                   int block, int chunk, uint32_t *workCtr, int32_t *ids, float *d, int32_t *nf, uint32_t *ovfList,
                    uint32_t *ovfCount, StackEntry *deep, uint32_t *err, cudaStream_t s)
 {
   if (stack <= 32)
-    return launch_seg_knn<K, TIE, 32>(bvhs, poff, points, queries, skeys, order, nq, k, maxSqr, block, chunk, workCtr,
-                                      ids, d, nf, ovfList, ovfCount, deep, err, s);
+    return launch_seg_knn<K, TIE, 32>(bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, block, chunk,
+                                      workCtr, ids, d, nf, ovfList, ovfCount, deep, err, s);
   if (stack <= 64)
-    return launch_seg_knn<K, TIE, 64>(bvhs, poff, points, queries, skeys, order, nq, k, maxSqr, block, chunk, workCtr,
-                                      ids, d, nf, ovfList, ovfCount, deep, err, s);
-  return launch_seg_knn<K, TIE, 128>(bvhs, poff, points, queries, skeys, order, nq, k, maxSqr, block, chunk, workCtr,
-                                     ids, d, nf, ovfList, ovfCount, deep, err, s);
+    return launch_seg_knn<K, TIE, 64>(bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, block, chunk,
+                                      workCtr, ids, d, nf, ovfList, ovfCount, deep, err, s);
+  return launch_seg_knn<K, TIE, 128>(bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, block, chunk,
+                                     workCtr, ids, d, nf, ovfList, ovfCount, deep, err, s);
 }
 
 } // namespace
@@ -629,10 +687,10 @@ int batched_knn(const bq_bvh3f *bvhs, const uint32_t *poff, const float *points,
   const int tie = c.tieMode, st = c.stackDepth, b = c.blockSize;
 #define BQ_SEG_KNN(KK)                                                                                             \
   (tie == BQ_TIES_REFERENCE                                                                                        \
-       ? stack_dispatch<KK, TIE_REFERENCE>(st, bvhs, poff, points, queries, skeys, order, nq, k, maxSqr, b, chunk, \
-                                           ctl, ids, d, nf, ovfList, ctl + 1, deep, dErr, al.s)                    \
-       : stack_dispatch<KK, TIE_LOWEST>(st, bvhs, poff, points, queries, skeys, order, nq, k, maxSqr, b, chunk,    \
-                                        ctl, ids, d, nf, ovfList, ctl + 1, deep, dErr, al.s))
+       ? stack_dispatch<KK, TIE_REFERENCE>(st, bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, b, \
+                                           chunk, ctl, ids, d, nf, ovfList, ctl + 1, deep, dErr, al.s)                    \
+       : stack_dispatch<KK, TIE_LOWEST>(st, bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, b,    \
+                                        chunk, ctl, ids, d, nf, ovfList, ctl + 1, deep, dErr, al.s))
   int s;
   if (k <= 4) s = BQ_SEG_KNN(4);
   else if (k <= 8) s = BQ_SEG_KNN(8);

@@ -266,6 +266,45 @@ __host__ __device__ __forceinline__ uint32_t spread10(uint32_t x)
   return x;
 }
 
+// Position of a cell of the 1024^3 grid along a 3D Hilbert curve (30 bits;
+// Skilling, "Programming the Hilbert curve", 2004: undo the excess work of
+// each level, then Gray-encode).  Consecutive cells of this curve are
+// neighbours, so a run of queries ordered by it fills a compact box; a
+// Morton-ordered run jumps wherever it crosses a cell boundary of a high
+// level.
+__device__ __forceinline__ uint32_t hilbert30(uint32_t x, uint32_t y, uint32_t z)
+{
+#pragma unroll
+  for (uint32_t b = 512; b > 1; b >>= 1) {
+    const uint32_t m = b - 1;
+    if (x & b) x ^= m;
+    uint32_t t = (x ^ y) & m;
+    if (y & b) x ^= m;
+    else { x ^= t; y ^= t; }
+    t = (x ^ z) & m;
+    if (z & b) x ^= m;
+    else { x ^= t; z ^= t; }
+  }
+  y ^= x;
+  z ^= y;
+  uint32_t g = 0;
+#pragma unroll
+  for (uint32_t b = 512; b > 1; b >>= 1)
+    if (z & b) g ^= b - 1;
+  return (spread10(x ^ g) << 2) | (spread10(y ^ g) << 1) | spread10(z ^ g);
+}
+
+// key of a query in the visiting order: its cell in a cube over the tree's
+// root box (outside it, and NaN, clamp to the boundary cells)
+__device__ __forceinline__ uint32_t query_order_key(const float *__restrict__ rootBox, const float *__restrict__ q)
+{
+  const float lx = __ldg(rootBox), ly = __ldg(rootBox + 1), lz = __ldg(rootBox + 2);
+  const float ext = fmaxf(fmaxf(__ldg(rootBox + 3) - lx, __ldg(rootBox + 4) - ly), __ldg(rootBox + 5) - lz);
+  const float sc = 1024.0f / fmaxf(ext, 1e-20f);
+  return hilbert30(min(__float2uint_rz((q[0] - lx) * sc), 1023u), min(__float2uint_rz((q[1] - ly) * sc), 1023u),
+                   min(__float2uint_rz((q[2] - lz) * sc), 1023u));
+}
+
 // quantised cell as in the reference's Quantizer<float,D>::quantize
 // (cuBQL/builder/cuda/radix.h:55-62): float->uint truncation
 // (saturating, NaN -> 0), clamped to 2^bits - 1

@@ -5,7 +5,7 @@
 // cuBQL/queries/points/knn.h:75-116 findKNN) that user kernels call one
 // thread per query in input order.  Here one call answers a whole batch:
 //
-//   k_query_keys   30-bit Morton code of every query inside the root box
+//   k_query_keys   30-bit Hilbert position of every query in the root box
 //   onesweep sort  queries reordered along the curve (top 24 key bits),
 //                  so neighbouring threads walk nearly the same nodes
 //                  (L1/L2 reuse, less divergence)
@@ -13,11 +13,14 @@
 //                  one thread per query, shrinking-radius traversal with a
 //                  local-memory stack (bq_traverse.cuh); kNN keeps its
 //                  sorted top-k in registers
+//   k_knn_warp     kNN under the lowest-id rule: one search for the 32
+//                  queries of a warp (bq_group.cuh)
 //   *_deep         queries whose stack overflowed are re-run with a deep
 //                  stack in global memory instead of returning a wrong
 //                  answer (the reference returns early, :475-478)
 #include <algorithm>
 
+#include "bq_group.cuh"
 #include "bq_query.cuh"
 
 namespace bq {
@@ -39,14 +42,7 @@ __global__ void k_query_keys(const float *__restrict__ rootBox, const float *__r
   griddep_wait();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nq) return;
-  const float lx = __ldg(rootBox), ly = __ldg(rootBox + 1), lz = __ldg(rootBox + 2);
-  const float ext = fmaxf(fmaxf(__ldg(rootBox + 3) - lx, __ldg(rootBox + 4) - ly), __ldg(rootBox + 5) - lz);
-  const float sc = 1024.0f / fmaxf(ext, 1e-20f);
-  const float *q = queries + 3ull * t;
-  const uint32_t cx = min(__float2uint_rz((q[0] - lx) * sc), 1023u);
-  const uint32_t cy = min(__float2uint_rz((q[1] - ly) * sc), 1023u);
-  const uint32_t cz = min(__float2uint_rz((q[2] - lz) * sc), 1023u);
-  keys[t] = spread10(cx) | (spread10(cy) << 1) | (spread10(cz) << 2);
+  keys[t] = query_order_key(rootBox, queries + 3ull * t);
   idx[t] = t;
 }
 
@@ -125,9 +121,29 @@ struct KnnLeaf {
   }
 };
 
+template <int K, int TIE>
+__device__ __forceinline__ void write_knn(const KnnList<K, TIE> &list, uint32_t qi, int k, int32_t *outIds,
+                                          float *outD, int32_t *numFound)
+{
+  int found = 0;
+  int32_t *oi = outIds + (size_t)qi * k;
+  float *od = outD + (size_t)qi * k;
+#pragma unroll
+  for (int j = 0; j < K; j++) {
+    if (j >= K - k) {
+      const bool real = list.real(j);
+      oi[j - (K - k)] = real ? list.id(j) : -1;
+      od[j - (K - k)] = real ? list.dist(j) : INFINITY;
+      found += real ? 1 : 0;
+    }
+  }
+  if (numFound) numFound[qi] = found;
+}
+
+// seed: an upper bound of the k-th best squared distance (maxSqr: none)
 template <int K, int TIE, typename Stack>
 __device__ __forceinline__ bool run_knn(const Node *nodes, const uint32_t *primIDs, const float *points,
-                                        const float *queries, uint32_t qi, int k, float maxSqr, Stack &st,
+                                        const float *queries, uint32_t qi, int k, float maxSqr, float seed, Stack &st,
                                         int32_t *outIds, float *outD, int32_t *numFound)
 {
   const float *q = queries + 3ull * qi;
@@ -139,21 +155,41 @@ __device__ __forceinline__ bool run_knn(const Node *nodes, const uint32_t *primI
   leaf.qz = __ldg(q + 2);
   leaf.maxSqr = maxSqr;
   leaf.list.init(k);
-  if (!traverse<TIE>(nodes, leaf.qx, leaf.qy, leaf.qz, maxSqr, st, leaf)) return false;
-  int found = 0;
-  int32_t *oi = outIds + (size_t)qi * k;
-  float *od = outD + (size_t)qi * k;
-#pragma unroll
-  for (int j = 0; j < K; j++) {
-    if (j >= K - k) {
-      const bool real = leaf.list.real(j);
-      oi[j - (K - k)] = real ? leaf.list.id(j) : -1;
-      od[j - (K - k)] = real ? leaf.list.dist(j) : INFINITY;
-      found += real ? 1 : 0;
-    }
-  }
-  if (numFound) numFound[qi] = found;
+  if (!traverse<TIE>(nodes, leaf.qx, leaf.qy, leaf.qz, seed, st, leaf)) return false;
+  write_knn(leaf.list, qi, k, outIds, outD, numFound);
   return true;
+}
+
+// one search for the 32 queries of a warp; queries that cannot share it are
+// answered one thread each
+template <int K, int STACK>
+__global__ void __launch_bounds__(128, GroupShape<K>::BLOCKS) k_knn_warp(const Node *__restrict__ nodes, const uint32_t *__restrict__ primIDs,
+                                                  const float *__restrict__ points, const float *__restrict__ queries,
+                                                  const uint32_t *__restrict__ order, uint32_t nq, int k,
+                                                  float maxSqr, int32_t *__restrict__ outIds,
+                                                  float *__restrict__ outD, int32_t *__restrict__ numFound,
+                                                  uint32_t *__restrict__ ovfList, uint32_t *ovfCount)
+{
+  griddep_wait();
+  __shared__ GroupShared<K> sh[4];
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool alive = t < nq;
+  const uint32_t qi = order ? __ldg(order + min(t, nq - 1)) : min(t, nq - 1);
+  const float *q = queries + 3ull * qi;
+  const float qx = __ldg(q), qy = __ldg(q + 1), qz = __ldg(q + 2);
+  const bool in = alive && group_can_search(nodes, qx, qy, qz);
+  KnnList<K, TIE_LOWEST> list;
+  list.init(k);
+  const bool done = group_search<K>(nodes, primIDs, points, in, qx, qy, qz, maxSqr, list, sh[threadIdx.x >> 5]);
+  if (!alive) return;
+  if (done && in) {
+    write_knn(list, qi, k, outIds, outD, numFound);
+    return;
+  }
+  LocalStack<STACK> st;
+  if (!run_knn<K, TIE_LOWEST>(nodes, primIDs, points, queries, qi, k, maxSqr, in ? fminf(maxSqr, list.worst()) : maxSqr,
+                              st, outIds, outD, numFound))
+    ovfList[atomicAdd(ovfCount, 1u)] = qi;
 }
 
 template <int K, int TIE, int STACK>
@@ -170,7 +206,7 @@ __global__ void __launch_bounds__(128) k_knn(const Node *__restrict__ nodes, con
   const uint32_t qi = order ? __ldg(order + t) : t;
   extern __shared__ StackEntry sStack[];
   HybridStack<KNN_SMEM_STACK, STACK> st(sStack);
-  if (!run_knn<K, TIE>(nodes, primIDs, points, queries, qi, k, maxSqr, st, outIds, outD, numFound))
+  if (!run_knn<K, TIE>(nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD, numFound))
     ovfList[atomicAdd(ovfCount, 1u)] = qi;
 }
 
@@ -186,7 +222,7 @@ __global__ void k_knn_deep(const Node *__restrict__ nodes, const uint32_t *__res
   for (uint32_t w = tid; w < cnt; w += gridDim.x * blockDim.x) {
     const uint32_t qi = ovfList[w];
     GlobalStack st{stacks + (size_t)tid * DEEP_STACK, DEEP_STACK, 0};
-    if (!run_knn<K, TIE>(nodes, primIDs, points, queries, qi, k, maxSqr, st, outIds, outD, numFound)) {
+    if (!run_knn<K, TIE>(nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD, numFound)) {
       for (int j = 0; j < k; j++) {
         outIds[(size_t)qi * k + j] = -1;
         outD[(size_t)qi * k + j] = INFINITY;
@@ -380,9 +416,16 @@ void launch_knn(const bq_bvh3f *bvh, const float *points, const float *queries, 
   const Node *nodes = (const Node *)bvh->nodes;
   {
     ProfScope ps("query.knn", s);
-    launch_pdl(k_knn<K, TIE, STACK>, dim3(div_up(nq, block)), dim3(block),
-               KNN_SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries, qs.order, nq, k,
-               maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);
+    // The shared search needs an answer that does not depend on the visiting
+    // order, queries sorted along the curve and lists that fit its registers
+    // (k > 32 would need 246 a thread).
+    if (TIE == TIE_LOWEST && K <= 32 && qs.order && group_pays(nq, bvh->numPrims))
+      launch_pdl(k_knn_warp<K <= 32 ? K : 32, STACK>, dim3(div_up(nq, block)), dim3(block), 0, s, nodes, bvh->primIDs, points,
+                 queries, qs.order, nq, k, maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);
+    else
+      launch_pdl(k_knn<K, TIE, STACK>, dim3(div_up(nq, block)), dim3(block),
+                 KNN_SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries, qs.order, nq, k,
+                 maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);
   }
   ProfScope ps("query.deep", s);
   launch_pdl(k_knn_deep<K, TIE>, dim3(DEEP_THREADS / 128), dim3(128), 0, s, nodes, bvh->primIDs, points, queries, k,
