@@ -13,7 +13,7 @@
 
 #include <cuda/atomic>
 
-#include "bq_traverse.cuh"
+#include "bq_tri.cuh"
 
 namespace bq {
 int query_config(const bq_query_config *q, bq_query_config &out);
@@ -21,18 +21,6 @@ int query_config(const bq_query_config *q, bq_query_config &out);
 namespace {
 
 constexpr uint32_t BR_NO_PARENT = 0xffffffffu;
-constexpr int DEEP_THREADS = 2048;
-constexpr int DEEP_STACK = 1024;
-
-__device__ __forceinline__ uint32_t seg_find(const uint32_t *__restrict__ off, uint32_t numSegs, uint32_t i)
-{
-  uint32_t lo = 0, hi = numSegs;
-  while (hi - lo > 1) {
-    const uint32_t m = (lo + hi) >> 1;
-    if (__ldg(off + m) <= i) lo = m; else hi = m;
-  }
-  return lo;
-}
 
 // slot j of the node buffer belongs to the mesh whose block contains it;
 // returns false for slots past that tree's node count
@@ -112,63 +100,6 @@ __global__ void k_brefit_climb(Node *nodes, uint32_t numSlots, const bq_bvh3f *_
 // ------------------------------------------------------------------
 // batched closest triangle
 // ------------------------------------------------------------------
-struct V3 {
-  float x, y, z;
-};
-__device__ __forceinline__ V3 v3sub(V3 a, V3 b) { return V3{a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ float v3dot(V3 a, V3 b)
-{
-  float r = 0.f;
-  r += a.x * b.x;
-  r += a.y * b.y;
-  r += a.z * b.z;
-  return r;
-}
-__device__ __forceinline__ V3 v3cross(V3 a, V3 b)
-{
-  return V3{a.y * b.z - b.y * a.z, a.z * b.x - b.z * a.x, a.x * b.y - b.x * a.y};
-}
-__device__ __forceinline__ V3 ldv(const float *verts, int32_t i)
-{
-  const float *p = verts + 3ll * i;
-  return V3{__ldg(p), __ldg(p + 1), __ldg(p + 2)};
-}
-
-// the per-triangle test of bq_tri.cu (cuBQL/queries/triangles/findClosest.h:74-122)
-__device__ __forceinline__ void edge_cp(float &best, V3 &P, V3 a, V3 b, V3 p)
-{
-  const V3 ba = v3sub(b, a);
-  float t = v3dot(v3sub(p, a), ba) / v3dot(ba, ba);
-  t = fminf(fmaxf(t, 0.f), 1.f);
-  const V3 cp = V3{a.x + t * ba.x, a.y + t * ba.y, a.z + t * ba.z};
-  const V3 dv = v3sub(cp, p);
-  const float sd = v3dot(dv, dv);
-  if (sd >= best) return;
-  best = sd;
-  P = cp;
-}
-
-__device__ __forceinline__ float tri_cp(V3 a, V3 b, V3 c, V3 qp, V3 &P)
-{
-  float best = INFINITY;
-  V3 N = v3cross(v3sub(b, a), v3sub(c, a));
-  const bool outside = (N.x == 0.f && N.y == 0.f && N.z == 0.f) ||
-                       (v3dot(v3sub(qp, a), v3cross(v3sub(b, a), N)) >= 0.f) ||
-                       (v3dot(v3sub(qp, b), v3cross(v3sub(c, b), N)) >= 0.f) ||
-                       (v3dot(v3sub(qp, c), v3cross(v3sub(a, c), N)) >= 0.f);
-  if (outside) {
-    edge_cp(best, P, a, b, qp);
-    edge_cp(best, P, b, c, qp);
-    edge_cp(best, P, c, a, qp);
-    return best;
-  }
-  const float inv = 1.f / sqrtf(v3dot(N, N));
-  N = V3{N.x * inv, N.y * inv, N.z * inv};
-  const float sd = v3dot(v3sub(qp, a), N);
-  P = V3{qp.x - sd * N.x, qp.y - sd * N.y, qp.z - sd * N.z};
-  return sd * sd;
-}
-
 template <int TIE>
 struct BTriLeaf {
   const uint32_t *__restrict__ primIDs;  // mesh-local triangle ids
@@ -183,14 +114,14 @@ struct BTriLeaf {
     for (uint32_t j = 0; j < cnt; j++) {
       const uint32_t pid = __ldg(primIDs + o + j);
       const int32_t *t = tris + 3ull * pid;
-      V3 p;
-      const float d = tri_cp(ldv(verts, __ldg(t)), ldv(verts, __ldg(t + 1)), ldv(verts, __ldg(t + 2)), q, p);
+      const TriHit h = tri_cp(ldv(verts, __ldg(t)), ldv(verts, __ldg(t + 1)), ldv(verts, __ldg(t + 2)), q);
+      const float d = h.d;
       const bool take = (TIE == TIE_REFERENCE) ? (d < best)
                                                : (d < best || (d == best && id >= 0 && (int32_t)pid < id));
       if (take) {
         best = d;
         id = (int32_t)pid;
-        P = p;
+        P = h.P;
       }
     }
     return best;
@@ -258,6 +189,22 @@ __global__ void k_btri_deep(const bq_bvh3f *__restrict__ bvhs, const uint32_t *_
   }
 }
 
+// visiting order of the queries: mesh by mesh, along a Hilbert curve in the
+// mesh's root box (as many of its top bits as the mesh index leaves)
+__global__ void k_btri_keys(const bq_bvh3f *__restrict__ bvhs, const float *__restrict__ queries, uint32_t nq,
+                            const uint32_t *__restrict__ qoff, uint32_t numSegs, int segBits,
+                            uint32_t *__restrict__ keys, uint32_t *__restrict__ idx)
+{
+  griddep_wait();
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nq) return;
+  const uint32_t s = seg_find(qoff, numSegs, t);
+  const bq_bvh3f d = bvhs[s];
+  const uint32_t h = d.numNodes ? query_order_key((const float *)d.nodes, queries + 3ull * t) : 0;
+  keys[t] = (uint32_t)((((uint64_t)s << 30) | h) >> max(segBits - 2, 0));
+  idx[t] = t;
+}
+
 } // namespace
 
 int batched_refit(const bq_bvh3f *bvhs, const uint32_t *off, uint32_t numSegs, uint32_t numPrims, bq_node3f *nodes,
@@ -289,26 +236,49 @@ int batched_tri_closest(const bq_bvh3f *bvhs, const uint32_t *triOff, const int3
   uint32_t *ovfList = nullptr, *ctl = nullptr;
   StackEntry *deep = nullptr;
   BQ_TRY(tmp.get(&ovfList, nq));
-  BQ_TRY(tmp.get(&ctl, 2));
+  BQ_TRY(tmp.get(&ctl, 3));  // overflow count, error word, heavy count
   BQ_TRY(tmp.get(&deep, (size_t)DEEP_THREADS * DEEP_STACK));
-  BQ_CUDA(cudaMemsetAsync(ctl, 0, 8, al.s));
+  BQ_CUDA(cudaMemsetAsync(ctl, 0, 12, al.s));
   uint32_t *err = errOut ? errOut : ctl + 1;
   const int b = c.blockSize;
+  if (c.tieMode == BQ_TIES_LOWEST_ID) {
+    uint32_t *heavy = nullptr;
+    const uint32_t *order = nullptr;
+    BQ_TRY(tmp.get(&heavy, nq));
+    int segBits = 0;
+    while (segBits < 32 && (1ull << segBits) < numSegs) segBits++;
+    if (c.reorder && nq > 1) {
+      uint32_t *keys[2], *idx[2];
+      BQ_TRY(tmp.get(&keys[0], nq));
+      BQ_TRY(tmp.get(&keys[1], nq));
+      BQ_TRY(tmp.get(&idx[0], nq));
+      BQ_TRY(tmp.get(&idx[1], nq));
+      ProfScope ps("batch.query_keys", al.s);
+      launch_pdl(k_btri_keys, dim3(div_up(nq, 256)), dim3(256), 0, al.s, bvhs, queries, nq, qoff, numSegs, segBits,
+                 keys[0], idx[0]);
+      int sel = 0;
+      // order only: 24 bits (3 passes) while they leave the curve at least 16
+      BQ_TRY(onesweep_sort_u32(keys, idx, nq, nullptr, segBits <= 8 ? 8 - std::max(2 - segBits, 0) : 0,
+                               std::min(32, 30 + segBits), nullptr, &sel, err, al));
+      order = idx[sel];
+    }
+    const TriMesh m{nullptr, nullptr, bvhs, triOff, qoff, numSegs, nullptr, tris, verts};
+    launch_tri_group(m, queries, order, nq, maxSqr, ids, d, P, heavy, ctl + 2, ovfList, ctl, al.s);
+    ProfScope ps("tri.deep", al.s);
+    launch_pdl(k_btri_deep<TIE_LOWEST>, dim3(DEEP_THREADS / 128), dim3(128), 0, al.s, bvhs, triOff, qoff, numSegs, tris,
+               verts, queries, maxSqr, ids, d, P, ovfList, ctl, deep, err);
+    BQ_CUDA(cudaGetLastError());
+    return BQ_OK;
+  }
   ProfScope ps("batch.tri", al.s, 2);
 #define BQ_BTRI(TIE, ST)                                                                                           \
   k_btri<TIE, ST><<<div_up(nq, b), b, 0, al.s>>>(bvhs, triOff, qoff, numSegs, tris, verts, queries, nq, maxSqr, ids, \
                                                  d, P, ovfList, ctl);                                              \
   k_btri_deep<TIE><<<DEEP_THREADS / 128, 128, 0, al.s>>>(bvhs, triOff, qoff, numSegs, tris, verts, queries, maxSqr,  \
                                                          ids, d, P, ovfList, ctl, deep, err)
-  if (c.tieMode == BQ_TIES_REFERENCE) {
-    if (c.stackDepth == 32) { BQ_BTRI(TIE_REFERENCE, 32); }
-    else if (c.stackDepth == 64) { BQ_BTRI(TIE_REFERENCE, 64); }
-    else { BQ_BTRI(TIE_REFERENCE, 128); }
-  } else {
-    if (c.stackDepth == 32) { BQ_BTRI(TIE_LOWEST, 32); }
-    else if (c.stackDepth == 64) { BQ_BTRI(TIE_LOWEST, 64); }
-    else { BQ_BTRI(TIE_LOWEST, 128); }
-  }
+  if (c.stackDepth == 32) { BQ_BTRI(TIE_REFERENCE, 32); }
+  else if (c.stackDepth == 64) { BQ_BTRI(TIE_REFERENCE, 64); }
+  else { BQ_BTRI(TIE_REFERENCE, 128); }
 #undef BQ_BTRI
   BQ_CUDA(cudaGetLastError());
   return BQ_OK;

@@ -2,7 +2,8 @@
 //
 // Forward: cuBQL::triangles::findClosest (cuBQL/queries/triangles/
 // findClosest.h:132-152) over an indexed mesh, batched like the point
-// queries (Morton-ordered queries, local stack, deep-stack fallback).  The
+// queries (Hilbert-ordered; eight lanes a query under the lowest-id rule, see
+// bq_tri.cuh, a thread each under the reference's; deep-stack fallback).  The
 // per-triangle arithmetic follows findClosest.h:56-122 expression for
 // expression (edge projections with clamped t, the three edge-plane tests,
 // the normalised plane distance), so nvcc contracts it as it does the
@@ -19,97 +20,17 @@
 // bitwise reproducible.
 #include <algorithm>
 
-#include "bq_traverse.cuh"
+#include "bq_tri.cuh"
 
 namespace bq {
 namespace {
 
-constexpr int DEEP_THREADS = 2048;
-constexpr int DEEP_STACK = 1024;
 // stack entries a triangle-query thread keeps in shared memory (the top of
 // its traversal stack); the rest of the stack is in local memory.  Measured
 // on the 4M-query, 1.31M-triangle workload: 45.0 ms with none, 46.4 with 8,
 // 44.8 with 16 -- the kernel waits on its node and vertex loads, not on the
 // stack -- so none.
 constexpr int TRI_SMEM_STACK = 0;
-
-struct V3 {
-  float x, y, z;
-};
-__device__ __forceinline__ V3 v3sub(V3 a, V3 b) { return V3{a.x - b.x, a.y - b.y, a.z - b.z}; }
-// dot as the reference's accumulating loop (cuBQL/math/vec.h:459-466)
-__device__ __forceinline__ float v3dot(V3 a, V3 b)
-{
-  float r = 0.f;
-  r += a.x * b.x;
-  r += a.y * b.y;
-  r += a.z * b.z;
-  return r;
-}
-// cuBQL/math/vec.h:232-237
-__device__ __forceinline__ V3 v3cross(V3 a, V3 b)
-{
-  return V3{a.y * b.z - b.y * a.z, a.z * b.x - b.z * a.x, a.x * b.y - b.x * a.y};
-}
-__device__ __forceinline__ V3 ldv(const float *verts, int32_t i)
-{
-  const float *p = verts + 3ll * i;
-  return V3{__ldg(p), __ldg(p + 1), __ldg(p + 2)};
-}
-
-// closest point on one triangle; region: 0 = inside (plane distance),
-// 1 = edge ab, 2 = edge bc, 3 = edge ca; t = parameter along that edge
-struct TriHit {
-  float d;
-  V3 P;
-  int region;
-  float t;
-};
-
-// Edge::closestPoint (findClosest.h:74-88)
-__device__ __forceinline__ void edge_cp(TriHit &h, V3 a, V3 b, V3 p, int region)
-{
-  const V3 ba = v3sub(b, a);
-  float t = v3dot(v3sub(p, a), ba) / v3dot(ba, ba);
-  t = fminf(fmaxf(t, 0.f), 1.f);
-  const V3 cp = V3{a.x + t * ba.x, a.y + t * ba.y, a.z + t * ba.z};
-  const V3 dv = v3sub(cp, p);
-  const float sd = v3dot(dv, dv);
-  if (sd >= h.d) return;
-  h.d = sd;
-  h.P = cp;
-  h.region = region;
-  h.t = t;
-}
-
-// closestPoint(result, triangle, qp) (findClosest.h:93-122), evaluated
-// against a running best starting at +inf
-__device__ __forceinline__ TriHit tri_cp(V3 a, V3 b, V3 c, V3 qp)
-{
-  TriHit h;
-  h.d = INFINITY;
-  h.P = V3{0.f, 0.f, 0.f};
-  h.region = -1;
-  h.t = 0.f;
-  V3 N = v3cross(v3sub(b, a), v3sub(c, a));
-  const bool outside = (N.x == 0.f && N.y == 0.f && N.z == 0.f) ||
-                       (v3dot(v3sub(qp, a), v3cross(v3sub(b, a), N)) >= 0.f) ||
-                       (v3dot(v3sub(qp, b), v3cross(v3sub(c, b), N)) >= 0.f) ||
-                       (v3dot(v3sub(qp, c), v3cross(v3sub(a, c), N)) >= 0.f);
-  if (outside) {
-    edge_cp(h, a, b, qp, 1);
-    edge_cp(h, b, c, qp, 2);
-    edge_cp(h, c, a, qp, 3);
-    return h;
-  }
-  const float inv = 1.f / sqrtf(v3dot(N, N));
-  N = V3{N.x * inv, N.y * inv, N.z * inv};
-  const float sd = v3dot(v3sub(qp, a), N);
-  h.d = sd * sd;
-  h.P = V3{qp.x - sd * N.x, qp.y - sd * N.y, qp.z - sd * N.z};
-  h.region = 0;
-  return h;
-}
 
 template <int TIE>
 struct TriLeaf {
@@ -180,6 +101,7 @@ __global__ void k_tri_deep(const Node *__restrict__ nodes, const uint32_t *__res
                            float *__restrict__ outD, float *__restrict__ outP, const uint32_t *ovfList,
                            const uint32_t *ovfCount, StackEntry *stacks, uint32_t *err)
 {
+  griddep_wait();
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t cnt = *ovfCount;
   for (uint32_t w = tid; w < cnt; w += gridDim.x * blockDim.x) {
@@ -223,14 +145,7 @@ __global__ void k_tri_keys(const Node *__restrict__ nodes, const float *__restri
 {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nq) return;
-  const Node root = ldg_node(nodes);
-  const float ext = fmaxf(fmaxf(root.a.w - root.a.x, root.b.x - root.a.y), root.b.y - root.a.z);
-  const float sc = 1024.0f / fmaxf(ext, 1e-20f);
-  const float *q = queries + 3ull * t;
-  const uint32_t cx = min(__float2uint_rz((q[0] - root.a.x) * sc), 1023u);
-  const uint32_t cy = min(__float2uint_rz((q[1] - root.a.y) * sc), 1023u);
-  const uint32_t cz = min(__float2uint_rz((q[2] - root.a.z) * sc), 1023u);
-  keys[t] = spread10(cx) | (spread10(cy) << 1) | (spread10(cz) << 2);
+  keys[t] = query_order_key((const float *)nodes, queries + 3ull * t);
   idx[t] = t;
 }
 
@@ -359,9 +274,9 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
   uint32_t *ovfList = nullptr, *ovfCount = nullptr, *order = nullptr;
   StackEntry *deep = nullptr;
   BQ_TRY(tmp.get(&ovfList, nq));
-  BQ_TRY(tmp.get(&ovfCount, 2));
+  BQ_TRY(tmp.get(&ovfCount, 3));  // overflow count, error word, heavy count
   BQ_TRY(tmp.get(&deep, (size_t)DEEP_THREADS * DEEP_STACK));
-  BQ_CUDA(cudaMemsetAsync(ovfCount, 0, 8, al.s));
+  BQ_CUDA(cudaMemsetAsync(ovfCount, 0, 12, al.s));
   uint32_t *err = ovfCount + 1;
   const Node *nodes = (const Node *)bvh->nodes;
   if (c.reorder && nq > 1) {
@@ -388,9 +303,22 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
     else if (c.stackDepth == 64) { BQ_TRI_LAUNCH(TIE_REFERENCE, 64); }
     else { BQ_TRI_LAUNCH(TIE_REFERENCE, 128); }
   } else {
-    if (c.stackDepth == 32) { BQ_TRI_LAUNCH(TIE_LOWEST, 32); }
-    else if (c.stackDepth == 64) { BQ_TRI_LAUNCH(TIE_LOWEST, 64); }
-    else { BQ_TRI_LAUNCH(TIE_LOWEST, 128); }
+    uint32_t *heavy = nullptr;
+    float4 *packed = nullptr;
+    BQ_TRY(tmp.get(&heavy, nq));
+    // a query tests some twenty triangles: the copy pays from about a
+    // twentieth as many queries as triangles
+    if ((uint64_t)nq * 16 >= bvh->numPrims) {
+      BQ_TRY(tmp.get(&packed, 3ull * bvh->numPrims));
+      ProfScope ps("tri.pack", al.s);
+      launch_pdl(k_tri_pack, dim3(div_up(bvh->numPrims, 256)), dim3(256), 0, al.s, bvh->primIDs, bvh->numPrims, tris,
+                 verts, packed);
+    }
+    const TriMesh m{nodes, bvh->primIDs, nullptr, nullptr, nullptr, 0, packed, tris, verts};
+    launch_tri_group(m, queries, order, nq, maxSqr, ids, d, P, heavy, ovfCount + 2, ovfList, ovfCount, al.s);
+    ProfScope ps("tri.deep", al.s);
+    launch_pdl(k_tri_deep<TIE_LOWEST>, dim3(DEEP_THREADS / 128), dim3(128), 0, al.s, nodes, bvh->primIDs, tris, verts,
+               queries, maxSqr, ids, d, P, ovfList, ovfCount, deep, err);
   }
 #undef BQ_TRI_LAUNCH
   BQ_CUDA(cudaGetLastError());

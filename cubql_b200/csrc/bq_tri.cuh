@@ -1,0 +1,434 @@
+// bq_tri.cuh -- closest triangle of a query by a group of lanes.
+//
+// A triangle query visits hundreds of nodes (inside a closed mesh most of
+// the surface is nearly equidistant) and tests few triangles, and
+// neighbouring queries need different numbers of steps: with one thread per
+// query five of a warp's 32 lanes were active on average, and the few
+// queries near the middle of a mesh kept their warps alive long after the
+// rest had finished.  Here G lanes share one query: they take G nodes at a
+// time off a stack in shared memory, push the children within the best
+// distance so far, and test up to G queued triangles at once.  A group goes
+// on to its next query as soon as one is answered, and starts it with the
+// triangle that the last one found (a neighbour's answer is nearly always
+// close), so culling works from the first step.  A query that takes more
+// than `limit` steps is left to a second launch with a whole warp each.
+//
+// 4M queries over 1.31M triangles: 50-57 ms with one thread per query (the
+// last warps ran alone for 20 ms), 22.8 ms so: 20.5 for the first launch,
+// bound by the L1 data pipe (89% of its wavefronts), 2.3 for the second.
+// Four lanes a query 23.5 ms, sixteen 32.9; one lane a child instead of a
+// pair of children 19.1 + 4.7 ms.  5,001 queries over the same mesh: 14.5
+// -> 0.9 ms.  A batch of 128 meshes, 6.4M queries: 19.3 -> 14.6 ms, of which
+// sorting the queries, which it did not do before, takes 0.6.
+//
+// The answer, the lowest id among equal distances, does not depend on the
+// visiting order; the reference's tie rule keeps the per-thread traversal.
+#pragma once
+
+#include <algorithm>
+
+#include "bq_traverse.cuh"
+
+namespace bq {
+
+constexpr int DEEP_THREADS = 2048;  // threads of a deep-stack re-run kernel
+constexpr int DEEP_STACK = 1024;    // entries of 8 bytes per deep stack
+
+struct V3 {
+  float x, y, z;
+};
+__device__ __forceinline__ V3 v3sub(V3 a, V3 b) { return V3{a.x - b.x, a.y - b.y, a.z - b.z}; }
+// dot as the reference's accumulating loop (cuBQL/math/vec.h:459-466)
+__device__ __forceinline__ float v3dot(V3 a, V3 b)
+{
+  float r = 0.f;
+  r += a.x * b.x;
+  r += a.y * b.y;
+  r += a.z * b.z;
+  return r;
+}
+// cuBQL/math/vec.h:232-237
+__device__ __forceinline__ V3 v3cross(V3 a, V3 b)
+{
+  return V3{a.y * b.z - b.y * a.z, a.z * b.x - b.z * a.x, a.x * b.y - b.x * a.y};
+}
+__device__ __forceinline__ V3 ldv(const float *verts, int32_t i)
+{
+  const float *p = verts + 3ll * i;
+  return V3{__ldg(p), __ldg(p + 1), __ldg(p + 2)};
+}
+
+// closest point on one triangle; region: 0 = inside (plane distance),
+// 1 = edge ab, 2 = edge bc, 3 = edge ca; t = parameter along that edge
+struct TriHit {
+  float d;
+  V3 P;
+  int region;
+  float t;
+};
+
+// Edge::closestPoint (findClosest.h:74-88)
+__device__ __forceinline__ void edge_cp(TriHit &h, V3 a, V3 b, V3 p, int region)
+{
+  const V3 ba = v3sub(b, a);
+  float t = v3dot(v3sub(p, a), ba) / v3dot(ba, ba);
+  t = fminf(fmaxf(t, 0.f), 1.f);
+  const V3 cp = V3{a.x + t * ba.x, a.y + t * ba.y, a.z + t * ba.z};
+  const V3 dv = v3sub(cp, p);
+  const float sd = v3dot(dv, dv);
+  if (sd >= h.d) return;
+  h.d = sd;
+  h.P = cp;
+  h.region = region;
+  h.t = t;
+}
+
+// closestPoint(result, triangle, qp) (findClosest.h:93-122), evaluated
+// against a running best starting at +inf
+__device__ __forceinline__ TriHit tri_cp(V3 a, V3 b, V3 c, V3 qp)
+{
+  TriHit h;
+  h.d = INFINITY;
+  h.P = V3{0.f, 0.f, 0.f};
+  h.region = -1;
+  h.t = 0.f;
+  V3 N = v3cross(v3sub(b, a), v3sub(c, a));
+  const bool outside = (N.x == 0.f && N.y == 0.f && N.z == 0.f) ||
+                       (v3dot(v3sub(qp, a), v3cross(v3sub(b, a), N)) >= 0.f) ||
+                       (v3dot(v3sub(qp, b), v3cross(v3sub(c, b), N)) >= 0.f) ||
+                       (v3dot(v3sub(qp, c), v3cross(v3sub(a, c), N)) >= 0.f);
+  if (outside) {
+    edge_cp(h, a, b, qp, 1);
+    edge_cp(h, b, c, qp, 2);
+    edge_cp(h, c, a, qp, 3);
+    return h;
+  }
+  const float inv = 1.f / sqrtf(v3dot(N, N));
+  N = V3{N.x * inv, N.y * inv, N.z * inv};
+  const float sd = v3dot(v3sub(qp, a), N);
+  h.d = sd * sd;
+  h.P = V3{qp.x - sd * N.x, qp.y - sd * N.y, qp.z - sd * N.z};
+  h.region = 0;
+  return h;
+}
+
+namespace {
+// ------------------------------------------------------------------
+// closest triangle, G lanes per query
+// ------------------------------------------------------------------
+constexpr int TRI_GROUP = 8;           // lanes of a query in the first launch
+constexpr int TRI_GROUP_STACK = 96;    // nodes on its stack
+constexpr int TRI_HEAVY_STACK = 1024;  // on a whole warp's, in the second
+// steps of the first launch; 4M queries, ms: 64 35.4, 192 25.4, 1024 27.2
+// (forward and adjoint); 5,001 queries: 1.10, 1.10, 1.51
+constexpr uint32_t TRI_STEP_LIMIT = 192;
+
+// One tree, or a batch of them.  `packed`: three float4 per triangle in leaf
+// order (the corners; the first one's w holds the id), or null, and corners
+// are fetched through the prim ids and index triples.
+struct TriMesh {
+  const Node *nodes;  // one tree
+  const uint32_t *primIDs;
+  const bq_bvh3f *bvhs;  // a batch (null: one tree)
+  const uint32_t *triOff, *queryOff;
+  uint32_t numSegs;
+  const float4 *packed;
+  const int32_t *tris;
+  const float *verts;
+};
+
+__device__ __forceinline__ uint32_t seg_find(const uint32_t *__restrict__ off, uint32_t numSegs, uint32_t i)
+{
+  uint32_t lo = 0, hi = numSegs;
+  while (hi - lo > 1) {
+    const uint32_t m = (lo + hi) >> 1;
+    if (__ldg(off + m) <= i) lo = m; else hi = m;
+  }
+  return lo;
+}
+
+// the triangle at leaf position `slot` of a tree whose first triangle is `base`
+__device__ __forceinline__ TriHit tri_test(const TriMesh &m, const uint32_t *primIDs, uint32_t base, uint32_t slot,
+                                           V3 q, int32_t &id)
+{
+  V3 a, b, c;
+  if (m.packed) {
+    const float4 *t = m.packed + 3ull * slot;
+    const float4 ta = __ldg(t), tb = __ldg(t + 1), tc = __ldg(t + 2);
+    a = V3{ta.x, ta.y, ta.z};
+    b = V3{tb.x, tb.y, tb.z};
+    c = V3{tc.x, tc.y, tc.z};
+    id = __float_as_int(ta.w);
+  } else {
+    id = (int32_t)(base + __ldg(primIDs + slot));
+    const int32_t *t = m.tris + 3ull * id;
+    a = ldv(m.verts, __ldg(t));
+    b = ldv(m.verts, __ldg(t + 1));
+    c = ldv(m.verts, __ldg(t + 2));
+  }
+  return tri_cp(a, b, c, q);
+}
+
+template <int G, int CAP>
+struct TriGroupShared {
+  StackEntry stack[CAP];
+  uint32_t queue[2 * G];
+};
+
+// The warp's 32 / G groups answer queries next(i), i = first .. last-1 of
+// their own.  HEAVY: the queries of the list left by the first launch, each
+// with the triangle it had found so far in outIds.
+template <int G, int CAP, bool HEAVY>
+__device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restrict__ queries,
+                                          const uint32_t *__restrict__ order, uint32_t at, uint32_t end,
+                                          uint32_t stride, float maxSqr, int32_t *outIds, float *outD, float *outP,
+                                          uint32_t *leftList, uint32_t *leftCount, TriGroupShared<G, CAP> &sh)
+{
+  const uint32_t gl = threadIdx.x & (G - 1);                  // lane of the group
+  const uint32_t shift = threadIdx.x & 31 & ~(uint32_t)(G - 1);  // the group's first lane
+  const uint32_t ones = G == 32 ? 0xffffffffu : (1u << G) - 1u;
+  const uint32_t below = (1u << gl) - 1u, above = (0xfffffffeu << gl) & ones;
+  auto ballot = [&](bool p) { return (__ballot_sync(0xffffffffu, p) >> shift) & ones; };
+  bool busy = false;
+  uint32_t qi = 0, sp = 0, qn = 0, steps = 0;
+  const Node *nodes = m.nodes;
+  const uint32_t *primIDs = m.primIDs;
+  uint32_t base = 0, seg = 0xffffffffu;
+  V3 q{0.f, 0.f, 0.f};
+  float best = 0.f;
+  int32_t id = -1, own = -2;       // best triangle of the group; the one whose point this lane holds
+  uint32_t slot = 0;               // where the best triangle is
+  V3 P{0.f, 0.f, 0.f};
+  uint32_t off0 = 0, cnt0 = 0, off1 = 0, cnt1 = 0;  // the leaves this lane found: nearer child, farther child
+  while (true) {
+    if (!busy && at < end) {
+      qi = order ? __ldg(order + at) : at;
+      at += stride;
+      const float *p = queries + 3ull * qi;
+      q = V3{__ldg(p), __ldg(p + 1), __ldg(p + 2)};
+      bool seeded = id >= 0;
+      if (m.bvhs) {
+        const uint32_t s = seg_find(m.queryOff, m.numSegs, qi);
+        seeded = seeded && s == seg;
+        seg = s;
+        const bq_bvh3f d = m.bvhs[s];
+        nodes = (const Node *)d.nodes;
+        primIDs = d.primIDs;
+        base = __ldg(m.triOff + s);
+        busy = d.numNodes != 0;
+      } else {
+        busy = true;
+      }
+      best = maxSqr;
+      id = -1;
+      own = -2;
+      steps = 0;
+      if (HEAVY) {  // the slot that the first launch left
+        slot = (uint32_t)outIds[qi];
+        seeded = slot != 0xffffffffu;
+      }
+      if (seeded) {
+        int32_t sid;
+        const TriHit h = tri_test(m, primIDs, base, slot, q, sid);
+        if (h.d < best) {
+          best = h.d;
+          id = sid;
+          own = gl == 0 ? sid : -2;
+          P = h.P;
+        }
+      }
+      if (busy) {
+        const uint64_t admin = ldg_admin(nodes);
+        if (admin_count(admin) == 0) {
+          if (gl == 0) sh.stack[0] = StackEntry{(uint32_t)admin_offset(admin), 0.f};
+          sp = 1;
+        } else if (gl == 0) {
+          off0 = (uint32_t)admin_offset(admin);
+          cnt0 = admin_count(admin);
+        }
+      } else if (gl == 0) {  // an empty tree
+        outIds[qi] = -1;
+        outD[qi] = INFINITY;
+        if (outP) outP[3ull * qi] = outP[3ull * qi + 1] = outP[3ull * qi + 2] = 0.f;
+      }
+    }
+    if (!__any_sync(0xffffffffu, busy || at < end)) return;
+    __syncwarp();
+    // take nodes; until a triangle is known nothing can be left out, so a
+    // narrow front keeps the stack short on the way down
+    const float reach = lowest_slack(best);
+    const uint32_t w = min(min(id >= 0 || best < 3e38f ? (uint32_t)G : 2u, sp), (uint32_t)CAP - sp);
+    const bool left = busy && sp != 0 && (w == 0 || (!HEAVY && ++steps > TRI_STEP_LIMIT));
+    bool act = busy && gl < w;
+    sp -= w;
+    StackEntry e{0, 0.f};
+    if (act) e = sh.stack[sp + w - 1 - gl];  // lane 0: the top
+    act = act && e.dist <= reach;
+    __syncwarp();  // the entries read are overwritten below
+    bool pushNear = false, pushFar = false;
+    StackEntry nearE{0, 0.f}, farE{0, 0.f};
+    if (act) {
+      const Node n0 = ldg_node(nodes + e.idx), n1 = ldg_node(nodes + e.idx + 1);
+      const float d0 = sqr_pbox(q.x, q.y, q.z, n0.a.x, n0.a.y, n0.a.z, n0.a.w, n0.b.x, n0.b.y);
+      const float d1 = sqr_pbox(q.x, q.y, q.z, n1.a.x, n1.a.y, n1.a.z, n1.a.w, n1.b.x, n1.b.y);
+      const uint64_t a0 = node_admin(n0), a1 = node_admin(n1);
+      const bool swap = d1 < d0;
+      const float dn = swap ? d1 : d0, df = swap ? d0 : d1;
+      const uint64_t an = swap ? a1 : a0, af = swap ? a0 : a1;
+      nearE = StackEntry{(uint32_t)admin_offset(an), dn};
+      farE = StackEntry{(uint32_t)admin_offset(af), df};
+      cnt0 = dn <= reach ? admin_count(an) : 0;
+      cnt1 = df <= reach ? admin_count(af) : 0;
+      pushNear = dn <= reach && cnt0 == 0;
+      pushFar = df <= reach && cnt1 == 0;
+      off0 = nearE.idx;
+      off1 = farE.idx;
+    }
+    const uint32_t mn = ballot(pushNear), mf = ballot(pushFar);
+    uint32_t to = sp + __popc(mn & above) + __popc(mf & above);
+    if (pushFar) sh.stack[to++] = farE;
+    if (pushNear) sh.stack[to] = nearE;
+    sp += __popc(mn) + __popc(mf);
+    // queue the triangles of the leaves found and test them: G at a time,
+    // or what there is when the group has nothing else to do or no bound
+    bool more = __any_sync(0xffffffffu, (cnt0 | cnt1) != 0 || (sp == 0 && qn != 0));
+    while (more) {
+      const bool has = (cnt0 | cnt1) != 0 && qn < G;
+      const uint32_t mh = ballot(has);
+      if (has) {
+        sh.queue[qn + __popc(mh & below)] = cnt0 ? off0 : off1;
+        if (cnt0) { off0++; cnt0--; }
+        else { off1++; cnt1--; }
+      }
+      qn += __popc(mh);
+      __syncwarp();
+      const uint32_t waiting = ballot((cnt0 | cnt1) != 0);
+      const bool due = qn >= G || (qn != 0 && waiting == 0 && (sp == 0 || id < 0));
+      if (__any_sync(0xffffffffu, due)) {
+        float td = INFINITY;
+        int32_t tid = 0x7fffffff;
+        TriHit h;
+        uint32_t sl = 0;
+        const uint32_t nb = min(qn, (uint32_t)G);
+        if (gl < nb) {
+          sl = sh.queue[gl];
+          h = tri_test(m, primIDs, base, sl, q, tid);
+          // below the best, or as near with a lower id
+          if (h.d < best || (h.d == best && id >= 0 && tid < id)) td = h.d;
+          else tid = 0x7fffffff;
+        }
+        const uint32_t rest = G + gl < qn ? sh.queue[G + gl] : 0;
+        float bd = td;
+        int32_t bi = tid;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+          const float od = __shfl_xor_sync(0xffffffffu, bd, o);
+          const int32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+          if (od < bd || (od == bd && oi < bi)) { bd = od; bi = oi; }
+        }
+        if (bi != 0x7fffffff) {
+          best = bd;
+          id = bi;
+          own = -2;
+          if (tid == bi) {
+            own = bi;
+            P = h.P;
+          }
+        }
+        const uint32_t from = __ffs(ballot(tid == bi)) - 1;  // the lane that tested it
+        const uint32_t ns = __shfl_sync(0xffffffffu, sl, from & (G - 1), G);
+        if (bi != 0x7fffffff) slot = ns;
+        __syncwarp();
+        if (G + gl < qn) sh.queue[gl] = rest;
+        qn -= nb;
+        __syncwarp();
+      }
+      more = __any_sync(0xffffffffu, (cnt0 | cnt1) != 0 || (sp == 0 && qn != 0));
+    }
+    if (busy && (left || sp == 0)) {
+      if (left && sp != 0) {
+        if (gl == 0) {
+          outIds[qi] = id >= 0 ? (int32_t)slot : -1;
+          leftList[atomicAdd(leftCount, 1u)] = qi;
+        }
+        // triangles still queued are found again
+      } else if (id >= 0 ? own == id : gl == 0) {
+        outIds[qi] = id;
+        outD[qi] = id >= 0 ? best : INFINITY;
+        if (outP) {
+          outP[3ull * qi] = id >= 0 ? P.x : 0.f;
+          outP[3ull * qi + 1] = id >= 0 ? P.y : 0.f;
+          outP[3ull * qi + 2] = id >= 0 ? P.z : 0.f;
+        }
+      }
+      busy = false;
+      sp = 0;
+      qn = 0;
+    }
+  }
+}
+
+// each group answers `run` queries next to each other in the visiting order
+__global__ void __launch_bounds__(128) k_tri_group(TriMesh m, const float *__restrict__ queries,
+                                                   const uint32_t *__restrict__ order, uint32_t nq, uint32_t run,
+                                                   float maxSqr, int32_t *outIds, float *outD, float *outP,
+                                                   uint32_t *leftList, uint32_t *leftCount)
+{
+  griddep_wait();
+  __shared__ TriGroupShared<TRI_GROUP, TRI_GROUP_STACK> sh[128 / TRI_GROUP];
+  const uint32_t g = threadIdx.x / TRI_GROUP;
+  const uint64_t at = ((uint64_t)blockIdx.x * (128 / TRI_GROUP) + g) * run;
+  const uint32_t b = (uint32_t)min(at, (uint64_t)nq), e = (uint32_t)min(at + run, (uint64_t)nq);
+  tri_group<TRI_GROUP, TRI_GROUP_STACK, false>(m, queries, order, b, e, 1, maxSqr, outIds, outD, outP, leftList,
+                                               leftCount, sh[g]);
+}
+
+__global__ void __launch_bounds__(128) k_tri_heavy(TriMesh m, const float *__restrict__ queries, float maxSqr,
+                                                   int32_t *outIds, float *outD, float *outP,
+                                                   const uint32_t *__restrict__ list, const uint32_t *listCount,
+                                                   uint32_t *leftList, uint32_t *leftCount)
+{
+  griddep_wait();
+  __shared__ TriGroupShared<32, TRI_HEAVY_STACK> sh[4];
+  const uint32_t warp = threadIdx.x >> 5;
+  tri_group<32, TRI_HEAVY_STACK, true>(m, queries, list, blockIdx.x * 4 + warp, *listCount, gridDim.x * 4, maxSqr,
+                                       outIds, outD, outP, leftList, leftCount, sh[warp]);
+}
+
+// queries a group answers one after the other: each but the first starts
+// from its neighbour's triangle, while every SM still gets its groups
+inline uint32_t tri_run(uint32_t nq) { return std::min(8u, std::max(1u, nq >> 17)); }
+
+// corners of every triangle in leaf order
+__global__ void k_tri_pack(const uint32_t *__restrict__ primIDs, uint32_t numPrims, const int32_t *__restrict__ tris,
+                           const float *__restrict__ verts, float4 *__restrict__ packed)
+{
+  griddep_wait();
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= numPrims) return;
+  const uint32_t id = __ldg(primIDs + j);
+  const int32_t *t = tris + 3ull * id;
+  const V3 a = ldv(verts, __ldg(t)), b = ldv(verts, __ldg(t + 1)), c = ldv(verts, __ldg(t + 2));
+  packed[3ull * j] = make_float4(a.x, a.y, a.z, __uint_as_float(id));
+  packed[3ull * j + 1] = make_float4(b.x, b.y, b.z, 0.f);
+  packed[3ull * j + 2] = make_float4(c.x, c.y, c.z, 0.f);
+}
+
+// the two launches; queries that neither finished are on ovfList.  heavy: a
+// list of nq words, count: two words, zeroed
+inline void launch_tri_group(const TriMesh &m, const float *queries, const uint32_t *order, uint32_t nq, float maxSqr,
+                             int32_t *ids, float *d, float *P, uint32_t *heavy, uint32_t *heavyCount,
+                             uint32_t *ovfList, uint32_t *ovfCount, cudaStream_t s)
+{
+  const uint32_t run = tri_run(nq);
+  {
+    ProfScope ps("tri.group", s);
+    launch_pdl(k_tri_group, dim3(div_up((uint64_t)div_up(nq, run) * TRI_GROUP, 128)), dim3(128), 0, s, m, queries,
+               order, nq, run, maxSqr, ids, d, P, heavy, heavyCount);
+  }
+  ProfScope ps("tri.heavy", s);
+  launch_pdl(k_tri_heavy, dim3(4 * num_sms()), dim3(128), 0, s, m, queries, maxSqr, ids, d, P,
+             (const uint32_t *)heavy, (const uint32_t *)heavyCount, ovfList, ovfCount);
+}
+} // namespace
+} // namespace bq

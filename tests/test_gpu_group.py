@@ -73,3 +73,54 @@ def test_batched_knn_warps_that_span_clouds(bq):
         a = bq.batched_knn(batch, tp, _cuda(off), tq, _cuda(qoff), k)
         b = bq.batched_knn(batch, tp, _cuda(off), tq, _cuda(qoff), k, qcfg=bq.query_config(reorder=0))
         assert _same(a, b), f"k {k}"
+
+
+def _mesh(level, n=None):
+    verts, tris = W.icosphere(level)
+    return _cuda(verts), _cuda(tris[:n])
+
+
+# sizes around a group of eight and a block's sixteen groups
+@pytest.mark.parametrize("nq", [1, 7, 8, 9, 129])
+@pytest.mark.parametrize("n", [1, 2, 80, 20480])
+def test_triangle_groups_do_not_depend_on_batch_or_tree(bq, n, nq):
+    """A query's answer is the same alone, among many (corners copied into
+    leaf order or fetched through the index), on a tree of another shape and
+    in a batch; and no farther than under the reference's rule."""
+    tv, tt = _mesh(5, n)
+    qs = _cuda(W.uniform_points(20000, W.SEED_QUERIES, -1.5, 1.5))
+    boxes = bq.triangles.boxes(tt, tv)
+    bvh, sah = bq.cuda.radixBuilder(boxes), bq.cuda.sahBuilder(boxes, bq.BuildConfig(makeLeafThreshold=3))
+    for r in (float("inf"), 0.05):
+        many = bq.triangles.findClosest(bvh, tt, tv, qs, maxSqrDist=r)
+        few = bq.triangles.findClosest(bvh, tt, tv, qs[:nq], maxSqrDist=r)
+        assert _same(few, [x[:nq] for x in many])
+        assert _same(bq.triangles.findClosest(sah, tt, tv, qs[:nq], maxSqrDist=r)[:2], few[:2])
+        ref = bq.triangles.findClosest(bvh, tt, tv, qs, maxSqrDist=r, qcfg=bq.query_config(tieMode=1))
+        assert bool((many[1] <= ref[1]).all()) and float((many[1] == ref[1]).float().mean()) > 0.99
+        off, qoff = _cuda(np.array([0, n, n])), _cuda(np.array([0, 20000, 20000]))
+        batch = bq.Batch(boxes, off)
+        for reorder in (0, 1):
+            got = bq.batched_tri_closest(batch, tt, tv, qs, qoff, maxSqrDist=r, qcfg=bq.query_config(reorder=reorder))
+            assert _same(got, many), f"batch, reorder {reorder}"
+
+
+def test_triangle_groups_heavy_queries(bq):
+    """Queries around the middle of a sphere of equal radius visit most of its
+    tree and go to the second launch; NaN and infinite ones find nothing."""
+    verts, tris = W.icosphere(6, amp=0.0)
+    tv, tt = _cuda(verts), _cuda(tris)
+    qs = W.uniform_points(300, 2, -0.02, 0.02)
+    qs[::17, 0] = np.nan
+    qs[5::17, 1] = np.inf
+    bvh = bq.cuda.radixBuilder(bq.triangles.boxes(tt, tv))
+    ids, d, p = (x.cpu().numpy() for x in bq.triangles.findClosest(bvh, tt, tv, _cuda(qs)))
+    ok = np.isfinite(qs).all(1)
+    assert (ids[~ok] == -1).all() and np.isinf(d[~ok]).all()
+    c = verts.astype(np.float64)[tris]
+    nrm = np.cross(c[:, 1] - c[:, 0], c[:, 2] - c[:, 0])
+    nrm /= np.linalg.norm(nrm, axis=1, keepdims=True)
+    for i in np.nonzero(ok)[0]:  # near the middle the closest point lies inside its triangle, on the nearest plane
+        h = np.abs((c[:, 0] * nrm).sum(1) - nrm @ qs[i].astype(np.float64)) ** 2
+        assert abs(d[i] - h.min()) <= 1e-6, i
+    assert np.allclose(((p[ok] - qs[ok]) ** 2).sum(1), d[ok], rtol=1e-5)
