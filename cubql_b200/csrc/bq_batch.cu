@@ -357,16 +357,17 @@ __device__ __forceinline__ void write_knn(const KnnList<K, TIE> &list, uint32_t 
 }
 
 // one search for a warp's 32 queries (bq_group.cuh), or one for each cloud
-// that they belong to; queries that cannot share it are answered one thread
-// each
-template <int K, int STACK>
+// that they belong to; queries that cannot share it go on a list (of places
+// in the visiting order), with what is known of their k-th best distance in
+// outD
+template <int K>
 __global__ void __launch_bounds__(128, GroupShape<K>::BLOCKS)
     k_seg_knn_warp(const bq_bvh3f *__restrict__ bvhs, const uint32_t *__restrict__ poff,
                    const float *__restrict__ points, const float *__restrict__ queries,
                    const uint32_t *__restrict__ qoff, const uint64_t *__restrict__ sortedKeys,
                    const uint32_t *__restrict__ order, uint32_t nq, int k, float maxSqr, int32_t *__restrict__ outIds,
-                   float *__restrict__ outD, int32_t *__restrict__ numFound, uint32_t *__restrict__ ovfList,
-                   uint32_t *ovfCount)
+                   float *__restrict__ outD, int32_t *__restrict__ numFound, uint32_t *__restrict__ leftList,
+                   uint32_t *leftCount)
 {
   griddep_wait();
   __shared__ GroupShared<K> sh[4];
@@ -376,35 +377,68 @@ __global__ void __launch_bounds__(128, GroupShape<K>::BLOCKS)
   const uint32_t qi = __ldg(order + tt);
   const uint32_t s = (uint32_t)(__ldg(sortedKeys + tt) >> 32);
   const float *q = queries + 3ull * qi;
-  BKnnLeaf<K, TIE_LOWEST> leaf;
-  leaf.qx = __ldg(q); leaf.qy = __ldg(q + 1); leaf.qz = __ldg(q + 2);
-  leaf.maxSqr = maxSqr;
-  leaf.list.init(k);
+  const float qx = __ldg(q), qy = __ldg(q + 1), qz = __ldg(q + 2);
+  KnnList<K, TIE_LOWEST> list;
+  list.init(k);
+  bool left = false;
   uint32_t todo = __ballot_sync(0xffffffffu, alive);
   while (todo) {
     const uint32_t s0 = __shfl_sync(0xffffffffu, s, __ffs(todo) - 1);
     const bool mine = alive && s == s0;
     todo &= ~__ballot_sync(0xffffffffu, mine);
     const bq_bvh3f d = bvhs[s0];
+    if (d.numNodes == 0) continue;  // no prims: the empty list is the answer
     const Node *nodes = (const Node *)d.nodes;
-    leaf.primIDs = d.primIDs;
-    leaf.points = points + 3ull * __ldg(poff + s0);
     bool in = false, done = false;
-    if (d.numNodes && group_pays(__ldg(qoff + s0 + 1) - __ldg(qoff + s0), d.numPrims)) {
-      in = mine && group_can_search(nodes, leaf.qx, leaf.qy, leaf.qz);
-      done = group_search<K>(nodes, d.primIDs, leaf.points, in, leaf.qx, leaf.qy, leaf.qz, maxSqr, leaf.list,
+    if (group_pays(__ldg(qoff + s0 + 1) - __ldg(qoff + s0), d.numPrims)) {
+      in = mine && group_can_search(nodes, qx, qy, qz);
+      done = group_search<K>(nodes, d.primIDs, points + 3ull * __ldg(poff + s0), in, qx, qy, qz, maxSqr, list,
                              sh[threadIdx.x >> 5]);
     }
-    if (mine && d.numNodes && !(done && in)) {
-      const float seed = in ? fminf(maxSqr, leaf.list.worst()) : maxSqr;
-      leaf.list.init(k);
-      LocalStack<STACK> st;
-      if (!traverse<TIE_LOWEST>(nodes, leaf.qx, leaf.qy, leaf.qz, seed, st, leaf)) ovfList[atomicAdd(ovfCount, 1u)] = t;
+    if (mine && !(done && in)) {
+      left = true;
+      outD[(size_t)qi * k] = in ? fminf(maxSqr, list.worst()) : maxSqr;
     }
-    __syncwarp();
   }
-  // (a query on the overflow list is written again by the deep-stack kernel)
-  if (alive) write_knn(leaf.list, qi, k, outIds, outD, numFound);
+  if (alive && !left) write_knn(list, qi, k, outIds, outD, numFound);
+  list_append(left, t, leftList, leftCount);
+}
+
+// the queries of that list, one thread each
+template <int K, int STACK>
+__global__ void __launch_bounds__(128) k_seg_knn_left(const bq_bvh3f *__restrict__ bvhs,
+                                                      const uint32_t *__restrict__ poff,
+                                                      const float *__restrict__ points,
+                                                      const float *__restrict__ queries,
+                                                      const uint64_t *__restrict__ sortedKeys,
+                                                      const uint32_t *__restrict__ order,
+                                                      const uint32_t *__restrict__ list, const uint32_t *listCount,
+                                                      int k, float maxSqr, int32_t *__restrict__ outIds, float *outD,
+                                                      int32_t *__restrict__ numFound, uint32_t *__restrict__ ovfList,
+                                                      uint32_t *ovfCount)
+{
+  griddep_wait();
+  const uint32_t cnt = *listCount;
+  for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < cnt; base += gridDim.x * blockDim.x) {
+    const bool alive = base + (threadIdx.x & 31) < cnt;
+    const uint32_t t = __ldg(list + min(base + (threadIdx.x & 31), cnt - 1));
+    const uint32_t qi = __ldg(order + t);
+    const uint32_t s = (uint32_t)(__ldg(sortedKeys + t) >> 32);
+    const bq_bvh3f d = bvhs[s];
+    const float *q = queries + 3ull * qi;
+    BKnnLeaf<K, TIE_LOWEST> leaf;
+    leaf.primIDs = d.primIDs;
+    leaf.points = points + 3ull * __ldg(poff + s);
+    leaf.qx = __ldg(q); leaf.qy = __ldg(q + 1); leaf.qz = __ldg(q + 2);
+    leaf.maxSqr = maxSqr;
+    leaf.list.init(k);
+    LocalStack<STACK> st;
+    const bool ok = traverse_warp<TIE_LOWEST>((const Node *)d.nodes, leaf.qx, leaf.qy, leaf.qz, outD[(size_t)qi * k],
+                                              st, leaf, alive);
+    if (!alive) continue;
+    if (ok) write_knn(leaf.list, qi, k, outIds, outD, numFound);
+    else ovfList[atomicAdd(ovfCount, 1u)] = t;
+  }
 }
 
 template <int K, int TIE, int STACK>
@@ -426,17 +460,12 @@ __global__ void __launch_bounds__(128) k_seg_knn(const bq_bvh3f *__restrict__ bv
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= nq) return;
     const uint32_t end = min(nq, base + (uint32_t)chunk);
-    for (uint32_t t = base + lane; t < end; t += 32) {
+    for (uint32_t first = base; first < end; first += 32) {  // no lane leaves early: the warp walks in step
+      const uint32_t t = min(first + lane, end - 1);
       const uint32_t qi = order ? __ldg(order + t) : t;
       const uint32_t s = (uint32_t)(__ldg(sortedKeys + t) >> 32);
       const bq_bvh3f d = bvhs[s];
-      int32_t *oi = outIds + (size_t)qi * k;
-      float *od = outD + (size_t)qi * k;
-      if (d.numNodes == 0) {
-        for (int j = 0; j < k; j++) { oi[j] = -1; od[j] = INFINITY; }
-        if (numFound) numFound[qi] = 0;
-        continue;
-      }
+      const bool alive = first + lane < end;
       const float *q = queries + 3ull * qi;
       BKnnLeaf<K, TIE> leaf;
       leaf.primIDs = d.primIDs;
@@ -445,7 +474,10 @@ __global__ void __launch_bounds__(128) k_seg_knn(const bq_bvh3f *__restrict__ bv
       leaf.maxSqr = maxSqr;
       leaf.list.init(k);
       LocalStack<STACK> st;
-      if (!traverse<TIE>((const Node *)d.nodes, leaf.qx, leaf.qy, leaf.qz, maxSqr, st, leaf)) {
+      const bool ok = traverse_warp<TIE>((const Node *)d.nodes, leaf.qx, leaf.qy, leaf.qz, maxSqr, st, leaf,
+                                         alive && d.numNodes != 0);
+      if (!alive) continue;
+      if (!ok) {
         ovfList[atomicAdd(ovfCount, 1u)] = t;
         continue;
       }
@@ -504,12 +536,16 @@ template <int K, int TIE, int STACK>
 int launch_seg_knn(const bq_bvh3f *bvhs, const uint32_t *poff, const float *points, const float *queries,
                    const uint32_t *qoff, const uint64_t *skeys, const uint32_t *order, uint32_t nq, int k, float maxSqr,
                    int block, int chunk, uint32_t *workCtr, int32_t *ids, float *d, int32_t *nf, uint32_t *ovfList,
-                   uint32_t *ovfCount, StackEntry *deep, uint32_t *err, cudaStream_t s)
+                   uint32_t *ovfCount, StackEntry *deep, uint32_t *leftList, uint32_t *err, cudaStream_t s)
 {
   if (TIE == TIE_LOWEST && K <= 32 && order) {
     ProfScope ps("batch.knn", s);
-    launch_pdl(k_seg_knn_warp<K <= 32 ? K : 32, STACK>, dim3(div_up(nq, block)), dim3(block), 0, s, bvhs, poff, points,
-               queries, qoff, skeys, order, nq, k, maxSqr, ids, d, nf, ovfList, ovfCount);
+    constexpr int KK = K <= 32 ? K : 32;
+    launch_pdl(k_seg_knn_warp<KK>, dim3(div_up(nq, block)), dim3(block), 0, s, bvhs, poff, points, queries, qoff,
+               skeys, order, nq, k, maxSqr, ids, d, nf, leftList, workCtr);
+    launch_pdl(k_seg_knn_left<KK, STACK>, dim3(std::min(div_up(nq, 128), 8 * num_sms())), dim3(128), 0, s, bvhs, poff,
+               points, queries, skeys, order, (const uint32_t *)leftList, (const uint32_t *)workCtr, k, maxSqr, ids, d,
+               nf, ovfList, ovfCount);
   } else {
     int perSm = 0;
     BQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_seg_knn<K, TIE, STACK>, block, 0));
@@ -529,16 +565,16 @@ template <int K, int TIE>
 int stack_dispatch(int stack, const bq_bvh3f *bvhs, const uint32_t *poff, const float *points, const float *queries,
                    const uint32_t *qoff, const uint64_t *skeys, const uint32_t *order, uint32_t nq, int k, float maxSqr,
                    int block, int chunk, uint32_t *workCtr, int32_t *ids, float *d, int32_t *nf, uint32_t *ovfList,
-                   uint32_t *ovfCount, StackEntry *deep, uint32_t *err, cudaStream_t s)
+                   uint32_t *ovfCount, StackEntry *deep, uint32_t *leftList, uint32_t *err, cudaStream_t s)
 {
   if (stack <= 32)
     return launch_seg_knn<K, TIE, 32>(bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, block, chunk,
-                                      workCtr, ids, d, nf, ovfList, ovfCount, deep, err, s);
+                                      workCtr, ids, d, nf, ovfList, ovfCount, deep, leftList, err, s);
   if (stack <= 64)
     return launch_seg_knn<K, TIE, 64>(bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, block, chunk,
-                                      workCtr, ids, d, nf, ovfList, ovfCount, deep, err, s);
+                                      workCtr, ids, d, nf, ovfList, ovfCount, deep, leftList, err, s);
   return launch_seg_knn<K, TIE, 128>(bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, block, chunk,
-                                     workCtr, ids, d, nf, ovfList, ovfCount, deep, err, s);
+                                     workCtr, ids, d, nf, ovfList, ovfCount, deep, leftList, err, s);
 }
 
 } // namespace
@@ -684,13 +720,15 @@ int batched_knn(const bq_bvh3f *bvhs, const uint32_t *poff, const float *points,
     order = idx[sel];
     skeys = keys[sel];
   }
+  // queries left by the shared search: the sort's other index buffer
+  uint32_t *leftList = c.reorder ? idx[sel ^ 1] : nullptr;
   const int tie = c.tieMode, st = c.stackDepth, b = c.blockSize;
 #define BQ_SEG_KNN(KK)                                                                                             \
   (tie == BQ_TIES_REFERENCE                                                                                        \
        ? stack_dispatch<KK, TIE_REFERENCE>(st, bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, b, \
-                                           chunk, ctl, ids, d, nf, ovfList, ctl + 1, deep, dErr, al.s)                    \
+                                           chunk, ctl, ids, d, nf, ovfList, ctl + 1, deep, leftList, dErr, al.s)                    \
        : stack_dispatch<KK, TIE_LOWEST>(st, bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, b,    \
-                                        chunk, ctl, ids, d, nf, ovfList, ctl + 1, deep, dErr, al.s))
+                                        chunk, ctl, ids, d, nf, ovfList, ctl + 1, deep, leftList, dErr, al.s))
   int s;
   if (k <= 4) s = BQ_SEG_KNN(4);
   else if (k <= 8) s = BQ_SEG_KNN(8);

@@ -112,7 +112,8 @@ __device__ __forceinline__ bool group_search(const Node *__restrict__ nodes, con
               lz = warp_min_f(in ? qz : INFINITY);
   const float hx = warp_max_f(in ? qx : -INFINITY), hy = warp_max_f(in ? qy : -INFINITY),
               hz = warp_max_f(in ? qz : -INFINITY);
-  // a prim is wanted at up to `mine`: below the radius, and no farther than the k-th best (at the same distance its id decides)
+  // a prim is wanted at up to `mine`: below the radius, and no farther than
+  // the k-th best (at the same distance its id decides)
   const float limit = maxSqr > 0.f ? __uint_as_float(__float_as_uint(maxSqr) - 1) : -1.f;
   float mine = in ? fminf(limit, list.worst()) : -1.f;
   auto warp_reach = [&]() {
@@ -173,7 +174,6 @@ __device__ __forceinline__ bool group_search(const Node *__restrict__ nodes, con
       __syncwarp();
       if (32 + lane < nq) sh.queue[lane] = rest;
       nq -= nb;
-      tested += nb;
       const uint32_t before = np;
       uint32_t merged = 0;
 #pragma unroll 1
@@ -192,17 +192,21 @@ __device__ __forceinline__ bool group_search(const Node *__restrict__ nodes, con
           merge_pending();
         }
       }
+      tested += nb;
       wanted += __reduce_add_sync(0xffffffffu, np + merged - before);
       reach = warp_reach();
       bounded = reach < 3e38f;
       __syncwarp();
     }
     if (sp == 0) break;  // the queue is empty too
-    // fewer than one lane wanted each prim that was tested: the queries
-    // are too far apart for one search.  (64 clouds, half of them clusters
-    // that most queries are far from: 10.2 ms with this, 13.4 when warps go
-    // on to 10,000 tests and 21.1 without a limit.)
-    if (tested > 512 + 16 * K && wanted < tested) return false;
+    // The queries are too far apart for one search when fewer than one lane
+    // wanted each prim that was tested, or far more prims were tested than a
+    // compact warp needs and not nearly every lane wanted them (copies of one
+    // point are wanted by all).  Queries far from the prims they look for are
+    // the case: without the second limit a warp tests thousands of prims.
+    // 2 clouds, one of them clusters: 1.22 ms with both, 2.76 with the first
+    // alone, 1.42 one thread per query; 512 clouds 69.8, 75.9, 83.8.
+    if (tested > 512 + 16 * K && wanted < (tested > 512 + 64 * K ? 8 : 1) * tested) return false;
     // Until k prims are known to every lane nothing can be left out: a
     // narrow front then keeps the stack short on the way down.
     const uint32_t w = min(min(bounded ? 16u : 4u, sp), (uint32_t)GROUP_STACK - sp);
@@ -241,12 +245,22 @@ __device__ __forceinline__ bool group_search(const Node *__restrict__ nodes, con
   return true;
 }
 
+// appends the flagged lanes' values to a list, in lane order (whole warp)
+__device__ __forceinline__ void list_append(bool flag, uint32_t value, uint32_t *list, uint32_t *count)
+{
+  const uint32_t m = __ballot_sync(0xffffffffu, flag), lane = threadIdx.x & 31;
+  uint32_t at = 0;
+  if (lane == 0 && m) at = atomicAdd(count, (uint32_t)__popc(m));
+  at = __shfl_sync(0xffffffffu, at, 0);
+  if (flag) list[at + __popc(m & ((1u << lane) - 1u))] = value;
+}
+
 // Whether the queries are dense enough among the prims for a warp's 32 to
 // share a search (a warp whose queries are not gives up by itself).  Below
 // this the box of 32 queries holds hundreds of prims that no lane wants:
-// 200,000 queries over 3M points, k = 16, take 1.95 ms shared and 1.36 ms
-// one thread each; 3,000 over 5M 4.3 and 0.44 ms; 1M over 2M, k = 32, 3.2
-// and 10.5 ms.
+// 200,000 queries over 3M points, k = 16, take 1.95 ms shared and 1.0 ms one
+// thread each; 3,000 over 5M 4.3 and 0.32 ms; 1M over 2M, k = 32, 3.7 and
+// 10.5 ms.
 __host__ __device__ inline bool group_pays(uint32_t numQueries, uint32_t numPrims)
 {
   return (uint64_t)numQueries * 8 >= numPrims;

@@ -141,8 +141,10 @@ __device__ __forceinline__ void write_knn(const KnnList<K, TIE> &list, uint32_t 
 }
 
 // seed: an upper bound of the k-th best squared distance (maxSqr: none)
-template <int K, int TIE, typename Stack>
-__device__ __forceinline__ bool run_knn(const Node *nodes, const uint32_t *primIDs, const float *points,
+// WARP: the whole warp calls together (lanes without a query: alive ==
+// false) and walks in step; otherwise one thread walks alone
+template <int K, int TIE, bool WARP, typename Stack>
+__device__ __forceinline__ bool run_knn(bool alive, const Node *nodes, const uint32_t *primIDs, const float *points,
                                         const float *queries, uint32_t qi, int k, float maxSqr, float seed, Stack &st,
                                         int32_t *outIds, float *outD, int32_t *numFound)
 {
@@ -155,41 +157,62 @@ __device__ __forceinline__ bool run_knn(const Node *nodes, const uint32_t *primI
   leaf.qz = __ldg(q + 2);
   leaf.maxSqr = maxSqr;
   leaf.list.init(k);
-  if (!traverse<TIE>(nodes, leaf.qx, leaf.qy, leaf.qz, seed, st, leaf)) return false;
+  if (WARP) {
+    const bool ok = traverse_warp<TIE>(nodes, leaf.qx, leaf.qy, leaf.qz, seed, st, leaf, alive);
+    if (!alive) return true;
+    if (!ok) return false;
+  } else if (!traverse<TIE>(nodes, leaf.qx, leaf.qy, leaf.qz, seed, st, leaf)) {
+    return false;
+  }
   write_knn(leaf.list, qi, k, outIds, outD, numFound);
   return true;
 }
 
-// one search for the 32 queries of a warp; queries that cannot share it are
-// answered one thread each
-template <int K, int STACK>
-__global__ void __launch_bounds__(128, GroupShape<K>::BLOCKS) k_knn_warp(const Node *__restrict__ nodes, const uint32_t *__restrict__ primIDs,
-                                                  const float *__restrict__ points, const float *__restrict__ queries,
-                                                  const uint32_t *__restrict__ order, uint32_t nq, int k,
-                                                  float maxSqr, int32_t *__restrict__ outIds,
-                                                  float *__restrict__ outD, int32_t *__restrict__ numFound,
-                                                  uint32_t *__restrict__ ovfList, uint32_t *ovfCount)
+// one search for the 32 queries of a warp; queries that cannot share it go
+// on a list, with what is known of their k-th best distance in outD
+template <int K>
+__global__ void __launch_bounds__(128, GroupShape<K>::BLOCKS)
+    k_knn_warp(const Node *__restrict__ nodes, const uint32_t *__restrict__ primIDs, const float *__restrict__ points,
+               const float *__restrict__ queries, const uint32_t *__restrict__ order, uint32_t nq, int k, float maxSqr,
+               int32_t *__restrict__ outIds, float *__restrict__ outD, int32_t *__restrict__ numFound,
+               uint32_t *__restrict__ leftList, uint32_t *leftCount)
 {
   griddep_wait();
   __shared__ GroupShared<K> sh[4];
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   const bool alive = t < nq;
-  const uint32_t qi = order ? __ldg(order + min(t, nq - 1)) : min(t, nq - 1);
+  const uint32_t qi = __ldg(order + min(t, nq - 1));
   const float *q = queries + 3ull * qi;
   const float qx = __ldg(q), qy = __ldg(q + 1), qz = __ldg(q + 2);
   const bool in = alive && group_can_search(nodes, qx, qy, qz);
   KnnList<K, TIE_LOWEST> list;
   list.init(k);
-  const bool done = group_search<K>(nodes, primIDs, points, in, qx, qy, qz, maxSqr, list, sh[threadIdx.x >> 5]);
-  if (!alive) return;
-  if (done && in) {
-    write_knn(list, qi, k, outIds, outD, numFound);
-    return;
+  const bool done = group_search<K>(nodes, primIDs, points, in, qx, qy, qz, maxSqr, list, sh[threadIdx.x >> 5]) && in;
+  if (alive && done) write_knn(list, qi, k, outIds, outD, numFound);
+  const bool left = alive && !done;
+  if (left) outD[(size_t)qi * k] = in ? fminf(maxSqr, list.worst()) : maxSqr;
+  list_append(left, qi, leftList, leftCount);
+}
+
+// the queries of that list, one thread each
+template <int K, int STACK>
+__global__ void __launch_bounds__(128) k_knn_left(const Node *__restrict__ nodes, const uint32_t *__restrict__ primIDs,
+                                                  const float *__restrict__ points, const float *__restrict__ queries,
+                                                  const uint32_t *__restrict__ list, const uint32_t *listCount, int k,
+                                                  float maxSqr, int32_t *__restrict__ outIds, float *outD,
+                                                  int32_t *__restrict__ numFound, uint32_t *__restrict__ ovfList,
+                                                  uint32_t *ovfCount)
+{
+  griddep_wait();
+  const uint32_t cnt = *listCount;
+  for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < cnt; base += gridDim.x * blockDim.x) {
+    const uint32_t t = base + (threadIdx.x & 31);
+    const uint32_t qi = __ldg(list + min(t, cnt - 1));
+    LocalStack<STACK> st;
+    if (!run_knn<K, TIE_LOWEST, true>(t < cnt, nodes, primIDs, points, queries, qi, k, maxSqr, outD[(size_t)qi * k],
+                                      st, outIds, outD, numFound))
+      ovfList[atomicAdd(ovfCount, 1u)] = qi;
   }
-  LocalStack<STACK> st;
-  if (!run_knn<K, TIE_LOWEST>(nodes, primIDs, points, queries, qi, k, maxSqr, in ? fminf(maxSqr, list.worst()) : maxSqr,
-                              st, outIds, outD, numFound))
-    ovfList[atomicAdd(ovfCount, 1u)] = qi;
 }
 
 template <int K, int TIE, int STACK>
@@ -202,11 +225,11 @@ __global__ void __launch_bounds__(128) k_knn(const Node *__restrict__ nodes, con
 {
   griddep_wait();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nq) return;
-  const uint32_t qi = order ? __ldg(order + t) : t;
+  const bool alive = t < nq;  // no early return: the warp walks in step
+  const uint32_t qi = order ? __ldg(order + min(t, nq - 1)) : min(t, nq - 1);
   extern __shared__ StackEntry sStack[];
   HybridStack<KNN_SMEM_STACK, STACK> st(sStack);
-  if (!run_knn<K, TIE>(nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD, numFound))
+  if (!run_knn<K, TIE, true>(alive, nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD, numFound))
     ovfList[atomicAdd(ovfCount, 1u)] = qi;
 }
 
@@ -222,7 +245,7 @@ __global__ void k_knn_deep(const Node *__restrict__ nodes, const uint32_t *__res
   for (uint32_t w = tid; w < cnt; w += gridDim.x * blockDim.x) {
     const uint32_t qi = ovfList[w];
     GlobalStack st{stacks + (size_t)tid * DEEP_STACK, DEEP_STACK, 0};
-    if (!run_knn<K, TIE>(nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD, numFound)) {
+    if (!run_knn<K, TIE, false>(true, nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD, numFound)) {
       for (int j = 0; j < k; j++) {
         outIds[(size_t)qi * k + j] = -1;
         outD[(size_t)qi * k + j] = INFINITY;
@@ -419,9 +442,14 @@ void launch_knn(const bq_bvh3f *bvh, const float *points, const float *queries, 
     // The shared search needs an answer that does not depend on the visiting
     // order, queries sorted along the curve and lists that fit its registers
     // (k > 32 would need 246 a thread).
-    if (TIE == TIE_LOWEST && K <= 32 && qs.order && group_pays(nq, bvh->numPrims))
-      launch_pdl(k_knn_warp<K <= 32 ? K : 32, STACK>, dim3(div_up(nq, block)), dim3(block), 0, s, nodes, bvh->primIDs, points,
-                 queries, qs.order, nq, k, maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);
+    if (TIE == TIE_LOWEST && K <= 32 && qs.order && group_pays(nq, bvh->numPrims)) {
+      constexpr int KK = K <= 32 ? K : 32;
+      launch_pdl(k_knn_warp<KK>, dim3(div_up(nq, block)), dim3(block), 0, s, nodes, bvh->primIDs, points, queries,
+                 qs.order, nq, k, maxSqr, ids, d, nf, qs.leftList, qs.ovfCount + 2);
+      launch_pdl(k_knn_left<KK, STACK>, dim3(std::min(div_up(nq, 128), 8 * num_sms())), dim3(128), 0, s, nodes,
+                 bvh->primIDs, points, queries, (const uint32_t *)qs.leftList, (const uint32_t *)(qs.ovfCount + 2), k,
+                 maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);
+    }
     else
       launch_pdl(k_knn<K, TIE, STACK>, dim3(div_up(nq, block)), dim3(block),
                  KNN_SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries, qs.order, nq, k,
@@ -527,10 +555,10 @@ int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, boo
                     QueryScratch &qs)
 {
   BQ_TRY(tmp.get(&qs.ovfList, nq));
-  BQ_TRY(tmp.get(&qs.ovfCount, 2));
+  BQ_TRY(tmp.get(&qs.ovfCount, 3));  // overflow count, error word, count of queries left
   qs.err = qs.ovfCount + 1;
   BQ_TRY(tmp.get(&qs.deep, (size_t)DEEP_THREADS * DEEP_STACK));
-  BQ_CUDA(cudaMemsetAsync(qs.ovfCount, 0, 8, al.s));
+  BQ_CUDA(cudaMemsetAsync(qs.ovfCount, 0, 12, al.s));
   if (reorder && nq > 1) {
     uint32_t *keys[2], *idx[2];
     BQ_TRY(tmp.get(&keys[0], nq));
@@ -548,6 +576,7 @@ int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, boo
     const int loBit = nq <= (1u << 21) ? 14 : 6;
     BQ_TRY(onesweep_sort_u32(keys, idx, nq, nullptr, loBit, 30, nullptr, &sel, qs.err, al));
     qs.order = idx[sel];
+    qs.leftList = keys[sel];  // the sorted keys are of no further use
   }
   return BQ_OK;
 }

@@ -52,6 +52,7 @@ struct CpExclude {
 struct QueryScratch {
   uint32_t *order = nullptr;
   uint32_t *ovfList = nullptr, *ovfCount = nullptr, *err = nullptr;
+  uint32_t *leftList = nullptr;  // nq words (with `order` only)
   StackEntry *deep = nullptr;
 };
 

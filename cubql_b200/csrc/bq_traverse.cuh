@@ -175,6 +175,93 @@ __device__ __forceinline__ bool traverse(const Node *__restrict__ nodes, float q
   return traverse_counted<TIE>(nodes, qx, qy, qz, cull, stack, leaf, none);
 }
 
+// Pushed far children carry what the pop needs to go on without touching
+// the node again: an inner child's entry holds its children's offset; a
+// leaf's entry holds its own node index and the sign bit of the distance
+// (distances are >= +0), and its prim range is read when it is popped.
+template <typename Stack>
+__device__ __forceinline__ bool push_child(Stack &stack, uint32_t idx, uint64_t admin, float d)
+{
+  const bool isLeaf = admin_count(admin) != 0;
+  return stack.push(isLeaf ? idx : (uint32_t)admin_offset(admin), isLeaf ? -d : d);
+}
+
+// The same traversal, every lane's in the same order, by a whole warp in
+// step (lanes without a query: alive == false): each round either all lanes
+// at an inner node open it or, once as many lanes wait at a leaf, all of
+// those process their leaf.  A leaf that costs much (kNN inserts into its
+// list) is then paid for by many lanes at once: 10M kNN16 queries 32.7 ->
+// 25.4 ms (13 of 32 lanes active instead of 5), 1M under the reference's
+// rule 1.17 -> 1.12 ms; waiting for twice or half as many lanes 26.3, 25.8.
+// A cheap leaf is better taken at once (closest point 3.8 -> 4.9 ms), so
+// only kNN uses this.
+template <int TIE, typename Stack, typename Leaf>
+__device__ __forceinline__ bool traverse_warp(const Node *__restrict__ nodes, float qx, float qy, float qz,
+                                              float cull, Stack &stack, Leaf &leaf, bool alive)
+{
+  bool ok = true;
+  uint32_t off = 0, cnt = 0;
+  if (alive) {
+    const uint64_t admin = ldg_admin(nodes);
+    off = (uint32_t)admin_offset(admin);
+    cnt = admin_count(admin);
+  }
+  while (true) {
+    const uint32_t inner = __ballot_sync(0xffffffffu, alive && cnt == 0);
+    const uint32_t atLeaf = __ballot_sync(0xffffffffu, alive && cnt != 0);
+    if ((inner | atLeaf) == 0) return ok;
+    bool needPop = false;
+    if (__popc(atLeaf) >= __popc(inner)) {
+      if (alive && cnt != 0) {
+        cull = fminf(cull, leaf(off, cnt));
+        needPop = true;
+      }
+    } else if (alive && cnt == 0) {
+      const Node n0 = ldg_node(nodes + off);
+      const Node n1 = ldg_node(nodes + off + 1);
+      const float d0 = sqr_pbox(qx, qy, qz, n0.a.x, n0.a.y, n0.a.z, n0.a.w, n0.b.x, n0.b.y);
+      const float d1 = sqr_pbox(qx, qy, qz, n1.a.x, n1.a.y, n1.a.z, n1.a.w, n1.b.x, n1.b.y);
+      const float dmin = fminf(d0, d1), dmax = fmaxf(d0, d1);
+      const float cs = TIE == TIE_REFERENCE ? cull : lowest_slack(cull);
+      if (TIE == TIE_REFERENCE ? (dmin >= cull) : (dmin > cs)) {
+        needPop = true;
+      } else {
+        const bool near0 = d0 < d1;
+        const uint64_t nearAdmin = near0 ? node_admin(n0) : node_admin(n1);
+        const uint64_t farAdmin = near0 ? node_admin(n1) : node_admin(n0);
+        if (TIE == TIE_REFERENCE ? (dmax < cull) : (dmax <= cs)) {
+          if (!push_child(stack, near0 ? off + 1 : off, farAdmin, dmax)) {
+            ok = false;
+            alive = false;
+          }
+        }
+        off = (uint32_t)admin_offset(nearAdmin);
+        cnt = admin_count(nearAdmin);
+      }
+    }
+    if (needPop) {
+      const float cs = TIE == TIE_REFERENCE ? cull : lowest_slack(cull);
+      while (true) {
+        if (stack.empty()) {
+          alive = false;
+          break;
+        }
+        const StackEntry e = stack.pop();
+        if (fabsf(e.dist) <= cs) {
+          off = e.idx;
+          cnt = 0;
+          if (__float_as_int(e.dist) < 0) {
+            const uint64_t admin = ldg_admin(nodes + e.idx);
+            off = (uint32_t)admin_offset(admin);
+            cnt = admin_count(admin);
+          }
+          break;
+        }
+      }
+    }
+  }
+}
+
 // a leaf functor that also counts the prims it is handed
 template <typename Leaf>
 struct CountingLeaf {
