@@ -124,3 +124,22 @@ def test_triangle_groups_heavy_queries(bq):
         h = np.abs((c[:, 0] * nrm).sum(1) - nrm @ qs[i].astype(np.float64)) ** 2
         assert abs(d[i] - h.min()) <= 1e-6, i
     assert np.allclose(((p[ok] - qs[ok]) ** 2).sum(1), d[ok], rtol=1e-5)
+
+
+# one warp, parts of one, more than one; above 16,384 queries are sorted.  A row of 3 ids sends most queries to the
+# second traversal.
+@pytest.mark.parametrize("nq", [1, 31, 33, 129, 16385])
+@pytest.mark.parametrize("leaf", [1, 8])
+def test_box_queries_of_partial_warps_match_oracle(bq, oracle, nq, leaf):
+    pts = W.uniform_points(6000)
+    boxes = boxes_np(pts)
+    c = W.uniform_points(nq, 4, -0.1, 1.1)
+    h = np.float32(0.02) + np.float32(0.06) * W.uniform_points(nq, 5)
+    q = np.concatenate([c - h, c + h], 1)
+    bvh = bq.cuda.radixBuilder(_cuda(boxes), bq.BuildConfig(makeLeafThreshold=leaf))
+    n, pr = bvh.to_host()
+    ooff, oids = oracle.box_query(n, pr, boxes, q)
+    for cap in (None, 3, 0):
+        off, ids = bq.fixedBoxQuery.findPrims(bvh, _cuda(boxes), _cuda(q), slabCap=cap)
+        assert np.array_equal(off.cpu().numpy(), ooff) and np.array_equal(ids.cpu().numpy(), oids), f"slab {cap}"
+    assert np.array_equal(bq.fixedBoxQuery.count(bvh, _cuda(boxes), _cuda(q)).cpu().numpy(), np.diff(ooff))
