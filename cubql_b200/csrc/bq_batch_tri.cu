@@ -247,7 +247,7 @@ int batched_tri_closest(const bq_bvh3f *bvhs, const uint32_t *triOff, const int3
     BQ_TRY(tmp.get(&heavy, nq));
     int segBits = 0;
     while (segBits < 32 && (1ull << segBits) < numSegs) segBits++;
-    if (c.reorder && nq > 1) {
+    if (c.reorder && nq >= TRI_ORDER_MIN) {
       uint32_t *keys[2], *idx[2];
       BQ_TRY(tmp.get(&keys[0], nq));
       BQ_TRY(tmp.get(&keys[1], nq));

@@ -296,13 +296,15 @@ __device__ __forceinline__ uint32_t hilbert30(uint32_t x, uint32_t y, uint32_t z
 
 // key of a query in the visiting order: its cell in a cube over the tree's
 // root box (outside it, and NaN, clamp to the boundary cells)
+template <bool HILBERT = true>
 __device__ __forceinline__ uint32_t query_order_key(const float *__restrict__ rootBox, const float *__restrict__ q)
 {
   const float lx = __ldg(rootBox), ly = __ldg(rootBox + 1), lz = __ldg(rootBox + 2);
   const float ext = fmaxf(fmaxf(__ldg(rootBox + 3) - lx, __ldg(rootBox + 4) - ly), __ldg(rootBox + 5) - lz);
   const float sc = 1024.0f / fmaxf(ext, 1e-20f);
-  return hilbert30(min(__float2uint_rz((q[0] - lx) * sc), 1023u), min(__float2uint_rz((q[1] - ly) * sc), 1023u),
-                   min(__float2uint_rz((q[2] - lz) * sc), 1023u));
+  const uint32_t x = min(__float2uint_rz((q[0] - lx) * sc), 1023u), y = min(__float2uint_rz((q[1] - ly) * sc), 1023u),
+                 z = min(__float2uint_rz((q[2] - lz) * sc), 1023u);
+  return HILBERT ? hilbert30(x, y, z) : spread10(x) | (spread10(y) << 1) | (spread10(z) << 2);
 }
 
 // quantised cell as in the reference's Quantizer<float,D>::quantize

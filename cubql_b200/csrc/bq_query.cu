@@ -35,32 +35,52 @@ namespace {
 constexpr int SMEM_STACK = 8;
 constexpr int KNN_SMEM_STACK = 0;
 
+// Fewer queries than this are taken in the given order: the keys and the
+// sort cost 30-45 us, more than coherent warps save while the queries do not
+// fill the GPU.  Closest point, ms sorted and not: 1,001 queries 0.119 and
+// 0.083, 16,001 0.140 and 0.108, 150,001 0.177 and 0.154 (over 1M points,
+// leaves of eight: 0.225 and 0.198); 1M have to be sorted.  kNN, k = 8:
+// 1,001 0.149 and 0.124, 5,003 0.172 and 0.161, 16,001 equal, 50,001 0.205
+// and 0.313; the shared search needs the order, and with long lists it pays
+// from the start (k = 32, 1,001: 0.195 and 0.259).
+constexpr uint32_t CP_ORDER_MIN = 1u << 17;
+inline uint32_t knn_order_min(int k) { return k <= 8 ? 4096 : 2; }
+
 // rootBox: lower xyz, upper xyz (the first 24 bytes of a binary root node)
+template <bool HILBERT>
 __global__ void k_query_keys(const float *__restrict__ rootBox, const float *__restrict__ queries, uint32_t nq,
                              uint32_t *__restrict__ keys, uint32_t *__restrict__ idx)
 {
   griddep_wait();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nq) return;
-  keys[t] = query_order_key(rootBox, queries + 3ull * t);
+  keys[t] = query_order_key<HILBERT>(rootBox, queries + 3ull * t);
   idx[t] = t;
 }
 
-template <int TIE, typename Stack>
-__device__ __forceinline__ bool run_cp(const Node *nodes, const uint32_t *primIDs, const float *points,
+// STEP: the whole warp calls together (lanes without a query: alive ==
+// false) and walks in step; otherwise each thread walks alone
+template <int TIE, bool STEP, typename Stack>
+__device__ __forceinline__ bool run_cp(bool alive, const Node *nodes, const uint32_t *primIDs, const float *points,
                                        const float *queries, uint32_t qi, float maxSqr, Stack &st, int32_t *outIds,
                                        float *outD, CpExclude ex)
 {
   const float *q = queries + 3ull * qi;
   CPLeaf<TIE> leaf{primIDs, points, __ldg(q), __ldg(q + 1), __ldg(q + 2), maxSqr, -1,
                    ex.ids ? __ldg(ex.ids + qi) : -1, ex.self};
-  if (!traverse<TIE>(nodes, leaf.qx, leaf.qy, leaf.qz, maxSqr, st, leaf)) return false;
+  if (STEP) {
+    const bool ok = traverse_warp<TIE>(nodes, leaf.qx, leaf.qy, leaf.qz, maxSqr, st, leaf, alive);
+    if (!alive) return true;
+    if (!ok) return false;
+  } else if (!traverse<TIE>(nodes, leaf.qx, leaf.qy, leaf.qz, maxSqr, st, leaf)) {
+    return false;
+  }
   outIds[qi] = leaf.id;
   outD[qi] = leaf.id >= 0 ? leaf.best : INFINITY;
   return true;
 }
 
-template <int TIE, int STACK>
+template <int TIE, int STACK, bool STEP>
 __global__ void __launch_bounds__(128) k_closest(const Node *__restrict__ nodes, const uint32_t *__restrict__ primIDs,
                                                  const float *__restrict__ points, const float *__restrict__ queries,
                                                  const uint32_t *__restrict__ order, uint32_t nq, float maxSqr,
@@ -69,11 +89,12 @@ __global__ void __launch_bounds__(128) k_closest(const Node *__restrict__ nodes,
 {
   griddep_wait();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nq) return;
-  const uint32_t qi = order ? __ldg(order + t) : t;
+  if (!STEP && t >= nq) return;
+  const uint32_t tt = STEP ? min(t, nq - 1) : t;
+  const uint32_t qi = order ? __ldg(order + tt) : tt;
   extern __shared__ StackEntry sStack[];
   HybridStack<SMEM_STACK, STACK> st(sStack);
-  if (!run_cp<TIE>(nodes, primIDs, points, queries, qi, maxSqr, st, outIds, outD, ex))
+  if (!run_cp<TIE, STEP>(t < nq, nodes, primIDs, points, queries, qi, maxSqr, st, outIds, outD, ex))
     ovfList[atomicAdd(ovfCount, 1u)] = qi;
 }
 
@@ -89,7 +110,7 @@ __global__ void k_closest_deep(const Node *__restrict__ nodes, const uint32_t *_
   for (uint32_t w = tid; w < cnt; w += gridDim.x * blockDim.x) {
     const uint32_t qi = ovfList[w];
     GlobalStack st{stacks + (size_t)tid * DEEP_STACK, DEEP_STACK, 0};
-    if (!run_cp<TIE>(nodes, primIDs, points, queries, qi, maxSqr, st, outIds, outD, ex)) {
+    if (!run_cp<TIE, false>(true, nodes, primIDs, points, queries, qi, maxSqr, st, outIds, outD, ex)) {
       outIds[qi] = -1;
       outD[qi] = INFINITY;
       atomicOr(err, DEV_ERR_STACK);
@@ -424,7 +445,11 @@ void launch_cp(const bq_bvh3f *bvh, const float *points, const float *queries, u
   const Node *nodes = (const Node *)bvh->nodes;
   {
     ProfScope ps("query.closest", s);
-    launch_pdl(k_closest<TIE, STACK>, dim3(div_up(nq, block)), dim3(block), SMEM_STACK * sizeof(StackEntry) * block,
+    // Leaves of several prims are worth waiting for (1M points, leaves of up
+    // to 8, 2.8 prims a node: 0.581 -> 0.549 ms), short ones are not (up to
+    // 4, 1.3 a node: 0.522 -> 0.560; leaves of one: 3.8 -> 4.9).
+    const bool step = bvh->numPrims / 2 >= bvh->numNodes;
+    launch_pdl(step ? k_closest<TIE, STACK, true> : k_closest<TIE, STACK, false>, dim3(div_up(nq, block)), dim3(block), SMEM_STACK * sizeof(StackEntry) * block,
                s, nodes, bvh->primIDs, points, queries, qs.order, nq, maxSqr, ids, d, qs.ovfList, qs.ovfCount, ex);
   }
   ProfScope ps("query.deep", s);
@@ -551,8 +576,8 @@ __global__ void k_fill_empty(uint32_t nq, int k, int32_t *ids, float *d, int32_t
   if (numFound && t < nq) numFound[t] = 0;
 }
 
-int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, bool reorder, TempSet &tmp, Alloc &al,
-                    QueryScratch &qs)
+int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, bool reorder, bool hilbert, TempSet &tmp,
+                    Alloc &al, QueryScratch &qs)
 {
   BQ_TRY(tmp.get(&qs.ovfList, nq));
   BQ_TRY(tmp.get(&qs.ovfCount, 3));  // overflow count, error word, count of queries left
@@ -567,7 +592,8 @@ int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, boo
     BQ_TRY(tmp.get(&idx[1], nq));
     {
       ProfScope ps("query.keys", al.s);
-      launch_pdl(k_query_keys, dim3(div_up(nq, 256)), dim3(256), 0, al.s, rootBox, queries, nq, keys[0], idx[0]);
+      launch_pdl(hilbert ? k_query_keys<true> : k_query_keys<false>, dim3(div_up(nq, 256)), dim3(256), 0, al.s, rootBox,
+                 queries, nq, keys[0], idx[0]);
     }
     BQ_CUDA(cudaGetLastError());
     int sel = 0;
@@ -629,7 +655,7 @@ int closest_point(const bq_bvh3f *bvh, const float *points, const float *queries
   }
   TempSet tmp(al);
   QueryScratch qs;
-  BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0, tmp, al, qs));
+  BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0 && nq >= CP_ORDER_MIN, false, tmp, al, qs));
   const int tie = c.tieMode, st = c.stackDepth, b = c.blockSize;
   if (tie == BQ_TIES_REFERENCE) {
     if (st == 32) launch_cp<TIE_REFERENCE, 32>(bvh, points, queries, nq, maxSqr, b, ids, d, qs, al.s, ex);
@@ -658,7 +684,11 @@ int knn(const bq_bvh3f *bvh, const float *points, const float *queries, uint32_t
   }
   TempSet tmp(al);
   QueryScratch qs;
-  BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0, tmp, al, qs));
+  // one search for a warp's queries (launch_knn); its order is the curve
+  // without jumps
+  const bool shared =
+      c.tieMode == BQ_TIES_LOWEST_ID && k <= 32 && c.lanesPerQuery == 1 && group_pays(nq, bvh->numPrims);
+  BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0 && nq >= knn_order_min(k), shared, tmp, al, qs));
   const int tie = c.tieMode, st = c.stackDepth, b = c.blockSize;
   if (c.lanesPerQuery > 1) {
     if (k > c.lanesPerQuery) return set_error(BQ_ERR_INVALID_ARGUMENT, "lanesPerQuery must be at least k");

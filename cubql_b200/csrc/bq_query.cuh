@@ -59,8 +59,8 @@ struct QueryScratch {
 // Allocates the call's scratch from `tmp` and, with `reorder`, sorts the
 // queries along a 30-bit Morton curve inside rootBox (6 device floats:
 // lower xyz, upper xyz); qs.order is then the visiting order.
-int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, bool reorder, TempSet &tmp, Alloc &al,
-                    QueryScratch &qs);
+int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, bool reorder, bool hilbert, TempSet &tmp,
+                    Alloc &al, QueryScratch &qs);
 // Synchronises the stream and turns the device error word into a status.
 int finish_queries(QueryScratch &qs, Alloc &al);
 // ids = -1, d = +inf (and numFound = 0) for nq queries of k results

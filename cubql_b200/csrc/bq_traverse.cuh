@@ -193,8 +193,8 @@ __device__ __forceinline__ bool push_child(Stack &stack, uint32_t idx, uint64_t 
 // list) is then paid for by many lanes at once: 10M kNN16 queries 32.7 ->
 // 25.4 ms (13 of 32 lanes active instead of 5), 1M under the reference's
 // rule 1.17 -> 1.12 ms; waiting for twice or half as many lanes 26.3, 25.8.
-// A cheap leaf is better taken at once (closest point 3.8 -> 4.9 ms), so
-// only kNN uses this.
+// A cheap leaf is better taken at once (closest point over leaves of one
+// prim 3.8 -> 4.9 ms).
 template <int TIE, typename Stack, typename Leaf>
 __device__ __forceinline__ bool traverse_warp(const Node *__restrict__ nodes, float qx, float qy, float qz,
                                               float cull, Stack &stack, Leaf &leaf, bool alive)

@@ -279,7 +279,7 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
   BQ_CUDA(cudaMemsetAsync(ovfCount, 0, 12, al.s));
   uint32_t *err = ovfCount + 1;
   const Node *nodes = (const Node *)bvh->nodes;
-  if (c.reorder && nq > 1) {
+  if (c.reorder && nq >= TRI_ORDER_MIN) {
     uint32_t *keys[2], *idx[2];
     BQ_TRY(tmp.get(&keys[0], nq));
     BQ_TRY(tmp.get(&keys[1], nq));

@@ -420,7 +420,7 @@ int wide_closest_point(const bq_wide_bvh3f *bvh, int W, const float *points, con
   else launch_pdl(k_wide_root_box<8>, dim3(1), dim3(32), 0, al.s, slots, rootBox);
   BQ_CUDA(cudaGetLastError());
   QueryScratch qs;
-  BQ_TRY(prepare_queries(rootBox, queries, nq, c.reorder != 0, tmp, al, qs));
+  BQ_TRY(prepare_queries(rootBox, queries, nq, c.reorder != 0, false, tmp, al, qs));
   if (W == 2) dispatch_wide_cp<2>(c.tieMode, c.stackDepth, bvh, points, queries, nq, maxSqr, c.blockSize, ids, d, qs, al.s);
   else if (W == 4) dispatch_wide_cp<4>(c.tieMode, c.stackDepth, bvh, points, queries, nq, maxSqr, c.blockSize, ids, d, qs, al.s);
   else dispatch_wide_cp<8>(c.tieMode, c.stackDepth, bvh, points, queries, nq, maxSqr, c.blockSize, ids, d, qs, al.s);

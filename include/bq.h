@@ -117,7 +117,7 @@ typedef struct bq_query_config {
   int tieMode;       /* BQ_TIES_LOWEST_ID or BQ_TIES_REFERENCE */
   int stackDepth;    /* fast-path stack entries: 32, 64 or 128 (0 = 64) */
   int blockSize;     /* threads per block: 64..512 (0 = 128) */
-  int reorder;       /* 1 = process queries in Morton order, 0 = input order */
+  int reorder;       /* 1 = process queries along a space-filling curve (small batches: as given), 0 = as given */
   int queriesPerWarp;/* one thread per query; queries a warp takes per work grab in the
                         persistent batched kernel (multiple of 32, <= 1024; 0 = 32) */
   int lanesPerQuery; /* bq_knn_f3 only.  0 or 1: one thread per query, its top-k list in

@@ -143,3 +143,18 @@ def test_box_queries_of_partial_warps_match_oracle(bq, oracle, nq, leaf):
         off, ids = bq.fixedBoxQuery.findPrims(bvh, _cuda(boxes), _cuda(q), slabCap=cap)
         assert np.array_equal(off.cpu().numpy(), ooff) and np.array_equal(ids.cpu().numpy(), oids), f"slab {cap}"
     assert np.array_equal(bq.fixedBoxQuery.count(bvh, _cuda(boxes), _cuda(q)).cpu().numpy(), np.diff(ooff))
+
+
+@pytest.mark.parametrize("tie", [0, 1])
+@pytest.mark.parametrize("leaf", [1, 8, 60])
+def test_closest_point_where_sorting_begins(bq, tie, leaf):
+    """The last batch taken as given and the first ones sorted, with leaves
+    that are processed at once and in step."""
+    pts = W.uniform_points(30000)
+    tp = _cuda(pts)
+    qs = _cuda(W.uniform_points(131073, W.SEED_QUERIES, -0.1, 1.1))
+    bvh = bq.gpuBuilder(_cuda(boxes_np(pts)), bq.BuildConfig(makeLeafThreshold=leaf))
+    b = bq.points.findClosest(bvh, tp, qs, qcfg=bq.query_config(tieMode=tie, reorder=0))
+    for nq in (1, 33, 131071, 131072, 131073):
+        a = bq.points.findClosest(bvh, tp, qs[:nq], qcfg=bq.query_config(tieMode=tie))
+        assert _same(a, [x[:nq] for x in b]), nq
