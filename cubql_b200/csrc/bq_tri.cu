@@ -15,8 +15,8 @@
 //     d sqrDist / d q   =  2 (q - X)
 //     d sqrDist / d v_k = -2 w_k (q - X).
 // Per query the three vertex contributions become (vertexID, pair index)
-// records; a stable radix sort by vertex id groups them and one thread per
-// vertex sums its group in sorted order.  No float atomics: the result is
+// records; a stable radix sort by vertex id groups them and one thread (or, of
+// many pairs, one warp) per vertex sums its group in a fixed order.  No float atomics: the result is
 // bitwise reproducible.
 #include <algorithm>
 
@@ -31,6 +31,11 @@ namespace {
 // 44.8 with 16 -- the kernel waits on its node and vertex loads, not on the
 // stack -- so none.
 constexpr int TRI_SMEM_STACK = 0;
+// Pairs a vertex (on average) from which a warp sums them, adjoint in ms by
+// thread and by warp: 18 (4M queries, 655,362 vertices) 2.29 and 1.30, 800
+// 1.64 and 0.16, 24,000 46 and 1.16; but 10 (6.4M queries, 1.9M vertices)
+// 1.50 and 3.74.
+constexpr uint32_t BWD_WARP_PAIRS = 16;
 
 template <int TIE>
 struct TriLeaf {
@@ -214,17 +219,55 @@ __global__ void k_tri_bwd_pairs(const int32_t *__restrict__ tris, const float *_
   }
 }
 
+// first pair with key >= v
+__device__ __forceinline__ uint32_t first_pair(const uint32_t *__restrict__ sortedKeys, uint32_t numPairs, uint32_t v)
+{
+  uint32_t lo = 0, hi = numPairs;
+  while (lo < hi) {
+    const uint32_t m = lo + ((hi - lo) >> 1);
+    if (sortedKeys[m] < v) lo = m + 1; else hi = m;
+  }
+  return lo;
+}
+
+// One warp per vertex: lane l adds its pairs l, l + 32, ... in sorted order,
+// then the lanes are added pairwise; reproducible like the other, and with
+// shorter chains of additions.  For meshes with many queries a vertex, where
+// one thread's chain of dependent gathers is what takes the time.
+__global__ void k_tri_bwd_reduce_warp(const uint32_t *__restrict__ sortedKeys,
+                                      const uint32_t *__restrict__ sortedVals, uint32_t numPairs,
+                                      const float *__restrict__ contrib, uint32_t numVerts, float *__restrict__ gradV)
+{
+  const uint32_t v = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (v >= numVerts) return;
+  const uint32_t lo = first_pair(sortedKeys, numPairs, v), hi = first_pair(sortedKeys, numPairs, v + 1);
+  float sx = 0.f, sy = 0.f, sz = 0.f;
+  for (uint32_t j = lo + lane; j < hi; j += 32) {
+    const uint32_t p = sortedVals[j];
+    sx += contrib[3ull * p + 0];
+    sy += contrib[3ull * p + 1];
+    sz += contrib[3ull * p + 2];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sx += __shfl_xor_sync(0xffffffffu, sx, o);
+    sy += __shfl_xor_sync(0xffffffffu, sy, o);
+    sz += __shfl_xor_sync(0xffffffffu, sz, o);
+  }
+  if (lane == 0) {
+    gradV[3ull * v + 0] = sx;
+    gradV[3ull * v + 1] = sy;
+    gradV[3ull * v + 2] = sz;
+  }
+}
+
 __global__ void k_tri_bwd_reduce(const uint32_t *__restrict__ sortedKeys, const uint32_t *__restrict__ sortedVals,
                                  uint32_t numPairs, const float *__restrict__ contrib, uint32_t numVerts,
                                  float *__restrict__ gradV)
 {
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= numVerts) return;
-  uint32_t lo = 0, hi = numPairs;  // first pair with key >= v
-  while (lo < hi) {
-    uint32_t m = lo + ((hi - lo) >> 1);
-    if (sortedKeys[m] < v) lo = m + 1; else hi = m;
-  }
+  const uint32_t lo = first_pair(sortedKeys, numPairs, v);
   float sx = 0.f, sy = 0.f, sz = 0.f;
   for (uint32_t j = lo; j < numPairs && sortedKeys[j] == v; j++) {
     const uint32_t p = sortedVals[j];
@@ -359,7 +402,9 @@ int tri_distance_bwd(const int32_t *tris, const float *verts, uint32_t numVerts,
   while (bits < 32 && (1ull << bits) <= numVerts) bits++;
   int sel = 0;
   BQ_TRY(onesweep_sort_u32(keys, vals, np, nullptr, 0, bits, nullptr, &sel, err, al));
-  if (numVerts)
+  if (numVerts && np / BWD_WARP_PAIRS >= numVerts)
+    k_tri_bwd_reduce_warp<<<div_up(numVerts, 8), 256, 0, al.s>>>(keys[sel], vals[sel], np, contrib, numVerts, gradV);
+  else if (numVerts)
     k_tri_bwd_reduce<<<div_up(numVerts, 256), 256, 0, al.s>>>(keys[sel], vals[sel], np, contrib, numVerts, gradV);
   BQ_CUDA(cudaGetLastError());
   uint32_t herr = 0;

@@ -158,3 +158,18 @@ def test_closest_point_where_sorting_begins(bq, tie, leaf):
     for nq in (1, 33, 131071, 131072, 131073):
         a = bq.points.findClosest(bvh, tp, qs[:nq], qcfg=bq.query_config(tieMode=tie))
         assert _same(a, [x[:nq] for x in b]), nq
+
+
+# just below and above the pairs a vertex at which a warp sums them, and many more
+@pytest.mark.parametrize("nq", [250, 863, 864, 40000])
+def test_vertex_gradients_by_thread_and_by_warp(bq, oracle, nq):
+    verts, tris = W.icosphere(2)  # 162 vertices (below 16 pairs each up to 863 queries)
+    qs = W.uniform_points(nq, 3, -1.5, 1.5)
+    g = (0.5 + W.uniform_points(nq, 8)[:, 0]).astype(np.float32)
+    tv, tt, tq = _cuda(verts), _cuda(tris), _cuda(qs)
+    ids, _, _ = bq.triangles.findClosest(bq.cuda.radixBuilder(bq.triangles.boxes(tt, tv)), tt, tv, tq)
+    gq, gv = bq.triangles.distanceBackward(tt, tv, tq, ids, _cuda(g))
+    assert _same((gq, gv), bq.triangles.distanceBackward(tt, tv, tq, ids, _cuda(g)))
+    rq, rv = oracle.tri_grad_f64(tris, verts, qs, ids.cpu().numpy(), g)
+    # the bound the adjoint is held to elsewhere: 1e-5 of the norm
+    assert np.linalg.norm(gv.cpu().numpy() - rv) <= 1e-5 * np.linalg.norm(rv)
