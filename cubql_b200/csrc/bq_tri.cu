@@ -352,10 +352,14 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
     // a query tests some twenty triangles: the copy pays from about a
     // twentieth as many queries as triangles
     if ((uint64_t)nq * 16 >= bvh->numPrims) {
-      BQ_TRY(tmp.get(&packed, 3ull * bvh->numPrims));
-      ProfScope ps("tri.pack", al.s);
-      launch_pdl(k_tri_pack, dim3(div_up(bvh->numPrims, 256)), dim3(256), 0, al.s, bvh->primIDs, bvh->numPrims, tris,
-                 verts, packed);
+      if (tmp.get(&packed, 3ull * bvh->numPrims) != BQ_OK) {
+        packed = nullptr;  // no room for the copy: corners through the index
+        cudaGetLastError();
+      } else {
+        ProfScope ps("tri.pack", al.s);
+        launch_pdl(k_tri_pack, dim3(div_up(bvh->numPrims, 256)), dim3(256), 0, al.s, bvh->primIDs, bvh->numPrims, tris,
+                   verts, packed);
+      }
     }
     const TriMesh m{nodes, bvh->primIDs, nullptr, nullptr, nullptr, 0, packed, tris, verts};
     launch_tri_group(m, queries, order, nq, maxSqr, ids, d, P, heavy, ovfCount + 2, ovfList, ovfCount, al.s);
