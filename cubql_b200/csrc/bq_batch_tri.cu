@@ -100,46 +100,16 @@ __global__ void k_brefit_climb(Node *nodes, uint32_t numSlots, const bq_bvh3f *_
 // ------------------------------------------------------------------
 // batched closest triangle
 // ------------------------------------------------------------------
-template <int TIE>
-struct BTriLeaf {
-  const uint32_t *__restrict__ primIDs;  // mesh-local triangle ids
-  const int32_t *__restrict__ tris;      // this mesh's first triangle
-  const float *__restrict__ verts;
-  V3 q;
-  float best;
-  int32_t id;
-  V3 P;
-  __device__ __forceinline__ float operator()(uint64_t o, uint32_t cnt)
-  {
-    for (uint32_t j = 0; j < cnt; j++) {
-      const uint32_t pid = __ldg(primIDs + o + j);
-      const int32_t *t = tris + 3ull * pid;
-      const TriHit h = tri_cp(ldv(verts, __ldg(t)), ldv(verts, __ldg(t + 1)), ldv(verts, __ldg(t + 2)), q);
-      const float d = h.d;
-      const bool take = (TIE == TIE_REFERENCE) ? (d < best)
-                                               : (d < best || (d == best && id >= 0 && (int32_t)pid < id));
-      if (take) {
-        best = d;
-        id = (int32_t)pid;
-        P = h.P;
-      }
-    }
-    return best;
-  }
-};
-
 template <int TIE, typename Stack>
 __device__ __forceinline__ bool run_btri(const bq_bvh3f &d, const uint32_t triBase, const int32_t *tris,
                                          const float *verts, const float *queries, uint32_t qi, float maxSqr,
                                          Stack &st, int32_t *outIds, float *outD, float *outP)
 {
-  const float *qp = queries + 3ull * qi;
-  BTriLeaf<TIE> leaf{d.primIDs, tris + 3ull * triBase, verts, V3{__ldg(qp), __ldg(qp + 1), __ldg(qp + 2)}, maxSqr,
-                     -1, V3{0.f, 0.f, 0.f}};
-  if (d.numNodes && !traverse<TIE>((const Node *)d.nodes, leaf.q.x, leaf.q.y, leaf.q.z, maxSqr, st, leaf))
+  TriLeaf<TIE> leaf(d.primIDs, tris + 3ull * triBase, verts, queries + 3ull * qi, maxSqr);
+  if (d.numNodes && !traverse<TIE>((const Node *)d.nodes, leaf.q.x, leaf.q.y, leaf.q.z, leaf.cull(), st, leaf))
     return false;
   outIds[qi] = leaf.id >= 0 ? (int32_t)(triBase + leaf.id) : -1;
-  outD[qi] = leaf.id >= 0 ? leaf.best : INFINITY;
+  outD[qi] = leaf.d;
   if (outP) {
     outP[3ull * qi] = leaf.P.x;
     outP[3ull * qi + 1] = leaf.P.y;

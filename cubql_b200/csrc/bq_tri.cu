@@ -37,43 +37,15 @@ constexpr int TRI_SMEM_STACK = 0;
 // 1.50 and 3.74.
 constexpr uint32_t BWD_WARP_PAIRS = 16;
 
-template <int TIE>
-struct TriLeaf {
-  const uint32_t *__restrict__ primIDs;
-  const int32_t *__restrict__ tris;
-  const float *__restrict__ verts;
-  V3 q;
-  float best;
-  int32_t id;
-  V3 P;
-  __device__ __forceinline__ float operator()(uint64_t off, uint32_t cnt)
-  {
-    for (uint32_t j = 0; j < cnt; j++) {
-      const uint32_t pid = __ldg(primIDs + off + j);
-      const int32_t *t = tris + 3ull * pid;
-      const TriHit h = tri_cp(ldv(verts, __ldg(t)), ldv(verts, __ldg(t + 1)), ldv(verts, __ldg(t + 2)), q);
-      const bool take = (TIE == TIE_REFERENCE) ? (h.d < best)
-                                               : (h.d < best || (h.d == best && id >= 0 && (int32_t)pid < id));
-      if (take) {
-        best = h.d;
-        id = (int32_t)pid;
-        P = h.P;
-      }
-    }
-    return best;
-  }
-};
-
 template <int TIE, typename Stack>
 __device__ __forceinline__ bool run_tri(const Node *nodes, const uint32_t *primIDs, const int32_t *tris,
                                         const float *verts, const float *queries, uint32_t qi, float maxSqr,
                                         Stack &st, int32_t *outIds, float *outD, float *outP)
 {
-  const float *qp = queries + 3ull * qi;
-  TriLeaf<TIE> leaf{primIDs, tris, verts, V3{__ldg(qp), __ldg(qp + 1), __ldg(qp + 2)}, maxSqr, -1, V3{0.f, 0.f, 0.f}};
-  if (!traverse<TIE>(nodes, leaf.q.x, leaf.q.y, leaf.q.z, maxSqr, st, leaf)) return false;
+  TriLeaf<TIE> leaf(primIDs, tris, verts, queries + 3ull * qi, maxSqr);
+  if (!traverse<TIE>(nodes, leaf.q.x, leaf.q.y, leaf.q.z, leaf.cull(), st, leaf)) return false;
   outIds[qi] = leaf.id;
-  outD[qi] = leaf.id >= 0 ? leaf.best : INFINITY;
+  outD[qi] = leaf.d;
   if (outP) {
     outP[3ull * qi + 0] = leaf.P.x;
     outP[3ull * qi + 1] = leaf.P.y;
@@ -134,12 +106,10 @@ __global__ void __launch_bounds__(128) k_tri_visit_count(const Node *__restrict_
   VisitCount vc;
   uint32_t prims = 0;
   if (t < nq) {  // no early return: every lane takes part in the warp sum below
-    const float *qp = queries + 3ull * t;
-    TriLeaf<TIE> leaf{primIDs, tris, verts, V3{__ldg(qp), __ldg(qp + 1), __ldg(qp + 2)}, maxSqr, -1,
-                      V3{0.f, 0.f, 0.f}};
+    TriLeaf<TIE> leaf(primIDs, tris, verts, queries + 3ull * t, maxSqr);
     CountingLeaf<TriLeaf<TIE>> cl{leaf};
     LocalStack<128> st;
-    traverse_counted<TIE>(nodes, leaf.q.x, leaf.q.y, leaf.q.z, maxSqr, st, cl, vc);
+    traverse_counted<TIE>(nodes, leaf.q.x, leaf.q.y, leaf.q.z, leaf.cull(), st, cl, vc);
     prims = cl.prims;
   }
   add_visit_counts(vc.pairs, vc.admins, prims, out);

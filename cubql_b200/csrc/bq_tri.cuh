@@ -21,8 +21,10 @@
 // -> 0.9 ms.  A batch of 128 meshes, 6.4M queries: 19.3 -> 14.6 ms, of which
 // sorting the queries, which it did not do before, takes 0.6.
 //
-// The answer, the lowest id among equal distances, does not depend on the
-// visiting order; the reference's tie rule keeps the per-thread traversal.
+// The answer, the lowest id among equal distances, is a function of the query
+// and the triangles alone, not of the tree, the batch or the visiting order
+// (tri_reach, tri_key); the reference's tie rule keeps the per-thread
+// traversal.
 #pragma once
 
 #include <algorithm>
@@ -119,6 +121,88 @@ __device__ __forceinline__ TriHit tri_cp(V3 a, V3 b, V3 c, V3 qp)
   return h;
 }
 
+// Lowest-id rule: culling that rounding cannot upset.  A closest point is
+// computed as a + t * (b - a), off its triangle by up to sqrt(3) * 2^-24 *
+// (|point| + |b - a|) in distance, and a plane distance carries the error of
+// the normal, so a triangle can be nearer, as computed, than its own box.
+// With the relative slack of the point queries its node was then visited or
+// not according to what had been found before: of 1M queries 0.001 to 0.03
+// from corners of unit triangles up to 56 changed their triangle with the
+// batch.  So (1) nodes are visited up to the best distance plus TRI_ROUND of
+// the coordinates at hand (query and distance), which covers edges up to some
+// eight times as long; (2) a triangle that is nearer than its box by more
+// than that (a sliver's plane) competes at the least distance at which its
+// box is visited, and still reports its own.  Every box around a triangle is
+// then visited while the triangle could win, whatever came first:
+// tri_reach(tri_key(d, b)) >= b, and boxes of ancestors are no farther.
+constexpr float TRI_ROUND = 0x1p-20f;
+
+__device__ __forceinline__ float abs_max(V3 q) { return fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z)); }
+
+// squared distance up to which nodes are visited; qmax: abs_max(query)
+__device__ __forceinline__ float tri_reach(float best, float qmax)
+{
+  const float r = sqrtf(fmaxf(best, 0.f));
+  const float s = __fmaf_rn(TRI_ROUND, qmax + r, r);
+  return lowest_slack(s * s);
+}
+
+// squared distance at which a triangle competes that is computed to be at d
+// and whose box is at boxD
+__device__ __forceinline__ float tri_key(float d, float boxD, float qmax)
+{
+  if (!(d < boxD)) return d;  // NaN stays NaN
+  const float r = fmaxf(__fmaf_rn(-TRI_ROUND, qmax, sqrtf(boxD)), 0.f) * (1.f / (1.f + TRI_ROUND));
+  return fmaxf(d, r * r);
+}
+
+__device__ __forceinline__ float tri_key(const TriHit &h, V3 a, V3 b, V3 c, V3 q, float qmax)
+{
+  const float boxD = sqr_pbox(q.x, q.y, q.z, fminf(fminf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y),
+                              fminf(fminf(a.z, b.z), c.z), fmaxf(fmaxf(a.x, b.x), c.x), fmaxf(fmaxf(a.y, b.y), c.y),
+                              fmaxf(fmaxf(a.z, b.z), c.z));
+  return tri_key(h.d, boxD, qmax);
+}
+
+// leaf functor of the per-thread traversals over one tree
+template <int TIE>
+struct TriLeaf {
+  const uint32_t *__restrict__ primIDs;
+  const int32_t *__restrict__ tris;  // the tree's first triangle
+  const float *__restrict__ verts;
+  V3 q;
+  float best;  // of the triangles met so far (lowest-id rule: tri_key's)
+  int32_t id = -1;
+  V3 P = V3{0.f, 0.f, 0.f};
+  float d = INFINITY;  // distance of triangle `id`
+  float qmax = 0.f;
+  __device__ __forceinline__ TriLeaf(const uint32_t *p, const int32_t *t, const float *v, const float *qp, float maxSqr)
+      : primIDs(p), tris(t), verts(v), q(V3{__ldg(qp), __ldg(qp + 1), __ldg(qp + 2)}), best(maxSqr)
+  {
+    if (TIE != TIE_REFERENCE) qmax = abs_max(q);
+  }
+  __device__ __forceinline__ float cull() const { return TIE == TIE_REFERENCE ? best : tri_reach(best, qmax); }
+  __device__ __forceinline__ float operator()(uint64_t off, uint32_t cnt)
+  {
+    for (uint32_t j = 0; j < cnt; j++) {
+      const uint32_t pid = __ldg(primIDs + off + j);
+      const int32_t *t = tris + 3ull * pid;
+      const V3 a = ldv(verts, __ldg(t)), b = ldv(verts, __ldg(t + 1)), c = ldv(verts, __ldg(t + 2));
+      const TriHit h = tri_cp(a, b, c, q);
+      const float key = TIE == TIE_REFERENCE ? h.d : tri_key(h, a, b, c, q, qmax);
+      const bool take = (TIE == TIE_REFERENCE) ? (key < best)
+                                               : (key < best || (key == best && id >= 0 && (int32_t)pid < id));
+      if (take) {
+        best = key;
+        d = h.d;
+        id = (int32_t)pid;
+        P = h.P;
+      }
+    }
+    return cull();
+  }
+};
+
 namespace {
 // ------------------------------------------------------------------
 // closest triangle, G lanes per query
@@ -154,9 +238,10 @@ __device__ __forceinline__ uint32_t seg_find(const uint32_t *__restrict__ off, u
   return lo;
 }
 
-// the triangle at leaf position `slot` of a tree whose first triangle is `base`
+// the triangle at leaf position `slot` of a tree whose first triangle is
+// `base`; key: where it competes
 __device__ __forceinline__ TriHit tri_test(const TriMesh &m, const uint32_t *primIDs, uint32_t base, uint32_t slot,
-                                           V3 q, int32_t &id)
+                                           V3 q, float qmax, int32_t &id, float &key)
 {
   V3 a, b, c;
   if (m.packed) {
@@ -173,7 +258,9 @@ __device__ __forceinline__ TriHit tri_test(const TriMesh &m, const uint32_t *pri
     b = ldv(m.verts, __ldg(t + 1));
     c = ldv(m.verts, __ldg(t + 2));
   }
-  return tri_cp(a, b, c, q);
+  const TriHit h = tri_cp(a, b, c, q);
+  key = tri_key(h, a, b, c, q, qmax);
+  return h;
 }
 
 template <int G, int CAP>
@@ -202,10 +289,11 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
   const uint32_t *primIDs = m.primIDs;
   uint32_t base = 0, seg = 0xffffffffu;
   V3 q{0.f, 0.f, 0.f};
-  float best = 0.f;
-  int32_t id = -1, own = -2;       // best triangle of the group; the one whose point this lane holds
-  uint32_t slot = 0;               // where the best triangle is
-  V3 P{0.f, 0.f, 0.f};
+  float best = 0.f, reach = 0.f, qmax = 0.f;
+  int32_t id = -1;                 // best triangle of the group
+  uint32_t slot = 0;               // where it is
+  V3 P{0.f, 0.f, 0.f};             // the lane that tested it: its point and distance
+  float ownD = -1.f;               // (negative: another lane did)
   uint32_t off0 = 0, cnt0 = 0, off1 = 0, cnt1 = 0;  // the leaves this lane found: nearer child, farther child
   while (true) {
     if (!busy && at < end) {
@@ -213,6 +301,7 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
       at += stride;
       const float *p = queries + 3ull * qi;
       q = V3{__ldg(p), __ldg(p + 1), __ldg(p + 2)};
+      qmax = abs_max(q);
       bool seeded = id >= 0;
       if (m.bvhs) {
         const uint32_t s = seg_find(m.queryOff, m.numSegs, qi);
@@ -228,7 +317,7 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
       }
       best = maxSqr;
       id = -1;
-      own = -2;
+      ownD = -1.f;
       steps = 0;
       if (HEAVY) {  // the slot that the first launch left
         slot = (uint32_t)outIds[qi];
@@ -236,14 +325,16 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
       }
       if (seeded) {
         int32_t sid;
-        const TriHit h = tri_test(m, primIDs, base, slot, q, sid);
-        if (h.d < best) {
-          best = h.d;
+        float key;
+        const TriHit h = tri_test(m, primIDs, base, slot, q, qmax, sid, key);
+        if (key < best) {
+          best = key;
           id = sid;
-          own = gl == 0 ? sid : -2;
           P = h.P;
+          if (gl == 0) ownD = h.d;
         }
       }
+      reach = tri_reach(best, qmax);
       if (busy) {
         const uint64_t admin = ldg_admin(nodes);
         if (admin_count(admin) == 0) {
@@ -263,7 +354,6 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
     __syncwarp();
     // take nodes; until a triangle is known nothing can be left out, so a
     // narrow front keeps the stack short on the way down
-    const float reach = lowest_slack(best);
     const uint32_t w = min(min(id >= 0 || best < 3e38f ? (uint32_t)G : 2u, sp), (uint32_t)CAP - sp);
     const bool left = busy && sp != 0 && (w == 0 || (!HEAVY && ++steps > TRI_STEP_LIMIT));
     bool act = busy && gl < w;
@@ -319,9 +409,10 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
         const uint32_t nb = min(qn, (uint32_t)G);
         if (gl < nb) {
           sl = sh.queue[gl];
-          h = tri_test(m, primIDs, base, sl, q, tid);
+          float key;
+          h = tri_test(m, primIDs, base, sl, q, qmax, tid, key);
           // below the best, or as near with a lower id
-          if (h.d < best || (h.d == best && id >= 0 && tid < id)) td = h.d;
+          if (key < best || (key == best && id >= 0 && tid < id)) td = key;
           else tid = 0x7fffffff;
         }
         const uint32_t rest = G + gl < qn ? sh.queue[G + gl] : 0;
@@ -335,11 +426,12 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
         }
         if (bi != 0x7fffffff) {
           best = bd;
+          reach = tri_reach(bd, qmax);
           id = bi;
-          own = -2;
+          ownD = -1.f;
           if (tid == bi) {
-            own = bi;
             P = h.P;
+            ownD = h.d;
           }
         }
         const uint32_t from = __ffs(ballot(tid == bi)) - 1;  // the lane that tested it
@@ -359,9 +451,9 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
           leftList[atomicAdd(leftCount, 1u)] = qi;
         }
         // triangles still queued are found again
-      } else if (id >= 0 ? own == id : gl == 0) {
+      } else if (id >= 0 ? ownD >= 0.f : gl == 0) {
         outIds[qi] = id;
-        outD[qi] = id >= 0 ? best : INFINITY;
+        outD[qi] = id >= 0 ? ownD : INFINITY;
         if (outP) {
           outP[3ull * qi] = id >= 0 ? P.x : 0.f;
           outP[3ull * qi + 1] = id >= 0 ? P.y : 0.f;
@@ -376,7 +468,7 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
 }
 
 // each group answers `run` queries next to each other in the visiting order
-__global__ void __launch_bounds__(128) k_tri_group(TriMesh m, const float *__restrict__ queries,
+__global__ void __launch_bounds__(128, 8) k_tri_group(TriMesh m, const float *__restrict__ queries,
                                                    const uint32_t *__restrict__ order, uint32_t nq, uint32_t run,
                                                    float maxSqr, int32_t *outIds, float *outD, float *outP,
                                                    uint32_t *leftList, uint32_t *leftCount)

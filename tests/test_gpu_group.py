@@ -105,6 +105,62 @@ def test_triangle_groups_do_not_depend_on_batch_or_tree(bq, n, nq):
             assert _same(got, many), f"batch, reorder {reorder}"
 
 
+def _corners(n, rng):
+    """n fans of three unit triangles, each around a corner that is extreme in its mesh's box."""
+    verts, tris = [], []
+    for _ in range(n):
+        a = rng.uniform(0, 2 * np.pi) + np.arange(3) * 2 * np.pi / 3 + rng.uniform(-0.4, 0.4, 3)
+        apex, b = rng.uniform(-3, 3, 3), len(verts)
+        verts += [apex] + list(apex + np.stack([np.cos(a), np.sin(a), -rng.uniform(0.2, 1.0, 3)], 1))
+        tris += [[b, b + 1, b + 2], [b, b + 2, b + 3], [b, b + 3, b + 1]]
+    return np.array(verts, np.float32), np.array(tris, np.int32)
+
+
+def _near_queries(verts, tris, nq, rng):
+    """Queries 0.001 to 0.03 from random points of the triangles, most of them near a corner."""
+    w = rng.random((nq, 3)) ** 3
+    p = (verts[tris[rng.integers(0, len(tris), nq)]] * (w / w.sum(1, keepdims=True))[:, :, None]).sum(1)
+    u = rng.standard_normal((nq, 3))
+    return (p + u / np.linalg.norm(u, axis=1, keepdims=True) * rng.uniform(0.001, 0.03, (nq, 1))).astype(np.float32)
+
+
+@pytest.mark.parametrize("fans", [1, 4, 64])
+def test_triangle_rounded_below_its_box_does_not_depend_on_batch_or_tree(bq, fans):
+    """Near unit triangles a computed distance can lie below the distance of
+    the triangle's own box; the answer still is a function of query and mesh."""
+    rng = np.random.default_rng(fans)
+    verts, tris = _corners(fans, rng)
+    tv, tt, tq = _cuda(verts), _cuda(tris), _cuda(_near_queries(verts, tris, 1_000_000, rng))
+    boxes = bq.triangles.boxes(tt, tv)
+    bvh, sah = bq.cuda.radixBuilder(boxes), bq.cuda.sahBuilder(boxes, bq.BuildConfig(makeLeafThreshold=3))
+    many = bq.triangles.findClosest(bvh, tt, tv, tq)
+    few = [torch.cat(x) for x in zip(*[bq.triangles.findClosest(bvh, tt, tv, q) for q in tq.split(20_000)])]
+    assert _same(few, many), "split"
+    assert _same(bq.triangles.findClosest(bvh, tt, tv, tq, qcfg=bq.query_config(reorder=0)), many), "as given"
+    assert _same(bq.triangles.findClosest(sah, tt, tv, tq), many), "another tree"
+    batch, off = bq.Batch(boxes, _cuda(np.array([0, len(tris)]))), _cuda(np.array([0, len(tq)]))
+    assert _same(bq.batched_tri_closest(batch, tt, tv, tq, off), many), "batch"
+    assert bool((many[1] <= bq.triangles.findClosest(bvh, tt, tv, tq, qcfg=bq.query_config(tieMode=1))[1]).all())
+
+
+def test_triangle_slivers_do_not_depend_on_batch_or_tree(bq):
+    """The plane of a sliver is known to few digits: its computed distance
+    can be far from its box's, and it is still met in every order."""
+    rng = np.random.default_rng(9)
+    c = rng.uniform(-1, 1, (3000, 1, 3))
+    e = rng.standard_normal((3000, 1, 3)) * 0.3
+    v = c + e * np.array([0.0, 0.5, 1.0])[None, :, None] + rng.standard_normal((3000, 3, 3)) * 10.0 ** rng.uniform(-8, -2, (3000, 1, 1))
+    verts, tris = v.reshape(-1, 3).astype(np.float32), np.arange(9000, dtype=np.int32).reshape(-1, 3)
+    tv, tt, tq = _cuda(verts), _cuda(tris), _cuda(_near_queries(verts, tris, 400_000, rng))
+    boxes = bq.triangles.boxes(tt, tv)
+    bvh, sah = bq.cuda.radixBuilder(boxes), bq.cuda.sahBuilder(boxes, bq.BuildConfig(makeLeafThreshold=3))
+    many = bq.triangles.findClosest(bvh, tt, tv, tq)
+    few = [torch.cat(x) for x in zip(*[bq.triangles.findClosest(bvh, tt, tv, q) for q in tq.split(20_000)])]
+    assert bool((many[0] >= 0).all())
+    assert _same(few, many), "split"
+    assert _same(bq.triangles.findClosest(sah, tt, tv, tq), many), "another tree"
+
+
 def test_triangle_groups_heavy_queries(bq):
     """Queries around the middle of a sphere of equal radius visit most of its
     tree and go to the second launch; NaN and infinite ones find nothing."""
