@@ -206,9 +206,9 @@ int batched_tri_closest(const bq_bvh3f *bvhs, const uint32_t *triOff, const int3
   uint32_t *ovfList = nullptr, *ctl = nullptr;
   StackEntry *deep = nullptr;
   BQ_TRY(tmp.get(&ovfList, nq));
-  BQ_TRY(tmp.get(&ctl, 3));  // overflow count, error word, heavy count
+  BQ_TRY(tmp.get(&ctl, 4));  // overflow count, error word, heavy count, count left by the first launch
   BQ_TRY(tmp.get(&deep, (size_t)DEEP_THREADS * DEEP_STACK));
-  BQ_CUDA(cudaMemsetAsync(ctl, 0, 12, al.s));
+  BQ_CUDA(cudaMemsetAsync(ctl, 0, 16, al.s));
   uint32_t *err = errOut ? errOut : ctl + 1;
   const int b = c.blockSize;
   if (c.tieMode == BQ_TIES_LOWEST_ID) {
@@ -217,7 +217,9 @@ int batched_tri_closest(const bq_bvh3f *bvhs, const uint32_t *triOff, const int3
     BQ_TRY(tmp.get(&heavy, nq));
     int segBits = 0;
     while (segBits < 32 && (1ull << segBits) < numSegs) segBits++;
-    if (c.reorder && nq >= TRI_ORDER_MIN) {
+    // with few queries a mesh, order within a mesh saves less than it costs
+    // (5,000 meshes of 320 triangles, 20 queries each: 0.366 and 0.296 ms)
+    if (c.reorder && nq >= TRI_ORDER_MIN && nq / 256 >= numSegs) {
       uint32_t *keys[2], *idx[2];
       BQ_TRY(tmp.get(&keys[0], nq));
       BQ_TRY(tmp.get(&keys[1], nq));
@@ -233,7 +235,7 @@ int batched_tri_closest(const bq_bvh3f *bvhs, const uint32_t *triOff, const int3
       order = idx[sel];
     }
     const TriMesh m{nullptr, nullptr, bvhs, triOff, qoff, numSegs, nullptr, tris, verts};
-    launch_tri_group(m, queries, order, nq, maxSqr, ids, d, P, heavy, ctl + 2, ovfList, ctl, al.s);
+    launch_tri_group(m, 0, queries, order, nq, maxSqr, ids, d, P, heavy, ovfList, ctl, ctl + 2, ctl + 3, al.s);
     ProfScope ps("tri.deep", al.s);
     launch_pdl(k_btri_deep<TIE_LOWEST>, dim3(DEEP_THREADS / 128), dim3(128), 0, al.s, bvhs, triOff, qoff, numSegs, tris,
                verts, queries, maxSqr, ids, d, P, ovfList, ctl, deep, err);

@@ -245,16 +245,6 @@ __device__ __forceinline__ bool group_search(const Node *__restrict__ nodes, con
   return true;
 }
 
-// appends the flagged lanes' values to a list, in lane order (whole warp)
-__device__ __forceinline__ void list_append(bool flag, uint32_t value, uint32_t *list, uint32_t *count)
-{
-  const uint32_t m = __ballot_sync(0xffffffffu, flag), lane = threadIdx.x & 31;
-  uint32_t at = 0;
-  if (lane == 0 && m) at = atomicAdd(count, (uint32_t)__popc(m));
-  at = __shfl_sync(0xffffffffu, at, 0);
-  if (flag) list[at + __popc(m & ((1u << lane) - 1u))] = value;
-}
-
 // Whether the queries are dense enough among the prims for a warp's 32 to
 // share a search (a warp whose queries are not gives up by itself).  Below
 // this the box of 32 queries holds hundreds of prims that no lane wants:

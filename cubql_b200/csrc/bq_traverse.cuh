@@ -195,9 +195,10 @@ __device__ __forceinline__ bool push_child(Stack &stack, uint32_t idx, uint64_t 
 // rule 1.17 -> 1.12 ms; waiting for twice or half as many lanes 26.3, 25.8.
 // A cheap leaf is better taken at once (closest point over leaves of one
 // prim 3.8 -> 4.9 ms).
-template <int TIE, typename Stack, typename Leaf>
+// LIMITED: lanes that are not done after `rounds` rounds return false.
+template <int TIE, bool LIMITED = false, typename Stack, typename Leaf>
 __device__ __forceinline__ bool traverse_warp(const Node *__restrict__ nodes, float qx, float qy, float qz,
-                                              float cull, Stack &stack, Leaf &leaf, bool alive)
+                                              float cull, Stack &stack, Leaf &leaf, bool alive, uint32_t rounds = 0)
 {
   bool ok = true;
   uint32_t off = 0, cnt = 0;
@@ -210,6 +211,7 @@ __device__ __forceinline__ bool traverse_warp(const Node *__restrict__ nodes, fl
     const uint32_t inner = __ballot_sync(0xffffffffu, alive && cnt == 0);
     const uint32_t atLeaf = __ballot_sync(0xffffffffu, alive && cnt != 0);
     if ((inner | atLeaf) == 0) return ok;
+    if (LIMITED && rounds-- == 0) return ok && !alive;
     bool needPop = false;
     if (__popc(atLeaf) >= __popc(inner)) {
       if (alive && cnt != 0) {
@@ -260,6 +262,16 @@ __device__ __forceinline__ bool traverse_warp(const Node *__restrict__ nodes, fl
       }
     }
   }
+}
+
+// appends the flagged lanes' values to a list, in lane order (whole warp)
+__device__ __forceinline__ void list_append(bool flag, uint32_t value, uint32_t *list, uint32_t *count)
+{
+  const uint32_t m = __ballot_sync(0xffffffffu, flag), lane = threadIdx.x & 31;
+  uint32_t at = 0;
+  if (lane == 0 && m) at = atomicAdd(count, (uint32_t)__popc(m));
+  at = __shfl_sync(0xffffffffu, at, 0);
+  if (flag) list[at + __popc(m & ((1u << lane) - 1u))] = value;
 }
 
 // a leaf functor that also counts the prims it is handed

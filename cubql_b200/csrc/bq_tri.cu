@@ -287,9 +287,9 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
   uint32_t *ovfList = nullptr, *ovfCount = nullptr, *order = nullptr;
   StackEntry *deep = nullptr;
   BQ_TRY(tmp.get(&ovfList, nq));
-  BQ_TRY(tmp.get(&ovfCount, 3));  // overflow count, error word, heavy count
+  BQ_TRY(tmp.get(&ovfCount, 4));  // overflow count, error word, heavy count, count left by the first launch
   BQ_TRY(tmp.get(&deep, (size_t)DEEP_THREADS * DEEP_STACK));
-  BQ_CUDA(cudaMemsetAsync(ovfCount, 0, 12, al.s));
+  BQ_CUDA(cudaMemsetAsync(ovfCount, 0, 16, al.s));
   uint32_t *err = ovfCount + 1;
   const Node *nodes = (const Node *)bvh->nodes;
   if (c.reorder && nq >= TRI_ORDER_MIN) {
@@ -332,7 +332,8 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
       }
     }
     const TriMesh m{nodes, bvh->primIDs, nullptr, nullptr, nullptr, 0, packed, tris, verts};
-    launch_tri_group(m, queries, order, nq, maxSqr, ids, d, P, heavy, ovfCount + 2, ovfList, ovfCount, al.s);
+    launch_tri_group(m, bvh->numPrims, queries, order, nq, maxSqr, ids, d, P, heavy, ovfList, ovfCount, ovfCount + 2, ovfCount + 3,
+                     al.s);
     ProfScope ps("tri.deep", al.s);
     launch_pdl(k_tri_deep<TIE_LOWEST>, dim3(DEEP_THREADS / 128), dim3(128), 0, al.s, nodes, bvh->primIDs, tris, verts,
                queries, maxSqr, ids, d, P, ovfList, ovfCount, deep, err);

@@ -11,7 +11,13 @@
 // on to its next query as soon as one is answered, and starts it with the
 // triangle that the last one found (a neighbour's answer is nearly always
 // close), so culling works from the first step.  A query that takes more
-// than `limit` steps is left to a second launch with a whole warp each.
+// than TRI_STEP_LIMIT steps is left to a second launch with a whole warp each.
+//
+// Eight lanes are wasted on a query that needs few steps: one near the surface
+// of a small mesh, or any over a handful of triangles.  Large batches over
+// meshes of up to TRI_NEAR_PRIMS triangles therefore start with a thread a
+// query, the warps in step, for some rounds; the groups get what is left, each
+// query with the triangle found so far (figures at TRI_NEAR_PRIMS).
 //
 // 4M queries over 1.31M triangles: 50-57 ms with one thread per query (the
 // last warps ran alone for 20 ms), 22.8 ms so: 20.5 for the first launch,
@@ -213,6 +219,19 @@ constexpr int TRI_HEAVY_STACK = 1024;  // on a whole warp's, in the second
 // steps of the first launch; 4M queries, ms: 64 35.4, 192 25.4, 1024 27.2
 // (forward and adjoint); 5,001 queries: 1.10, 1.10, 1.51
 constexpr uint32_t TRI_STEP_LIMIT = 192;
+// Where a thread a query goes first, and for how many rounds.  1M queries, ms
+// by a thread alone, by groups alone, and with 256 rounds before the groups:
+// within 0.01 of the surface of 80 triangles 0.22 0.72 0.24, of 20,480 0.68
+// 1.59 0.59, of 81,920 1.37 2.03 1.05, of 327,680 3.28 2.90 2.24; in a cube
+// around the mesh 0.46 0.90 0.42, 7.1 3.43 3.25, 8.1 3.71 4.12, 14.1 4.64
+// 5.65.  So up to 2^17 triangles.  100,000 queries, 20,480 triangles, near
+// 0.25 0.30 0.22, around 4.2 0.55 0.68 (0.64 with 128 rounds).  128 meshes of
+// 2,000 to 100,000 triangles, a fitting step: groups alone 17.6, 128 rounds
+// 16.5, 256 14.2.
+constexpr uint32_t TRI_NEAR_PRIMS = 1u << 17;
+constexpr uint32_t TRI_NEAR_MIN = 1u << 16;
+inline uint32_t tri_near_rounds(uint32_t nq) { return nq < (1u << 18) ? 128 : 256; }
+constexpr int TRI_NEAR_STACK = 64;     // entries of a thread's stack in the first of them
 
 // One tree, or a batch of them.  `packed`: three float4 per triangle in leaf
 // order (the corners; the first one's w holds the id), or null, and corners
@@ -269,10 +288,45 @@ struct TriGroupShared {
   uint32_t queue[2 * G];
 };
 
-// The warp's 32 / G groups answer queries next(i), i = first .. last-1 of
-// their own.  HEAVY: the queries of the list left by the first launch, each
-// with the triangle it had found so far in outIds.
-template <int G, int CAP, bool HEAVY>
+// leaf functor of a thread that answers a query by itself
+struct TriNear {
+  const TriMesh &m;
+  const uint32_t *primIDs;
+  uint32_t base;
+  V3 q;
+  float qmax, best;
+  int32_t id = -1;
+  uint32_t slot = 0;
+  V3 P{0.f, 0.f, 0.f};
+  float d = INFINITY;
+  __device__ __forceinline__ TriNear(const TriMesh &m_, const uint32_t *p, uint32_t b, V3 q_, float maxSqr)
+      : m(m_), primIDs(p), base(b), q(q_), qmax(abs_max(q_)), best(maxSqr)
+  {
+  }
+  __device__ __forceinline__ float cull() const { return tri_reach(best, qmax); }
+  __device__ __forceinline__ float operator()(uint64_t off, uint32_t cnt)
+  {
+    for (uint32_t j = 0; j < cnt; j++) {
+      int32_t tid;
+      float key;
+      const TriHit h = tri_test(m, primIDs, base, (uint32_t)off + j, q, qmax, tid, key);
+      if (key < best || (key == best && id >= 0 && tid < id)) {
+        best = key;
+        d = h.d;
+        id = tid;
+        P = h.P;
+        slot = (uint32_t)off + j;
+      }
+    }
+    return cull();
+  }
+};
+
+// The warp's 32 / G groups answer queries at, at + stride, .. of `order`.
+// SEEDED: they come from the list of an earlier launch, each with the place
+// of the triangle it had found so far in outIds.  LIMIT: steps after which a
+// query is left (0: none).
+template <int G, int CAP, bool SEEDED, uint32_t LIMIT>
 __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restrict__ queries,
                                           const uint32_t *__restrict__ order, uint32_t at, uint32_t end,
                                           uint32_t stride, float maxSqr, int32_t *outIds, float *outD, float *outP,
@@ -319,19 +373,42 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
       id = -1;
       ownD = -1.f;
       steps = 0;
-      if (HEAVY) {  // the slot that the first launch left
-        slot = (uint32_t)outIds[qi];
-        seeded = slot != 0xffffffffu;
+      // the last query's triangle and (odd lanes) the one found before
+      uint32_t cand = slot;
+      if (SEEDED && (gl & 1)) {
+        cand = (uint32_t)outIds[qi];
+        seeded = cand != 0xffffffffu;
       }
+      TriHit h;
+      float key = INFINITY;
+      int32_t sid = 0x7fffffff;
       if (seeded) {
-        int32_t sid;
-        float key;
-        const TriHit h = tri_test(m, primIDs, base, slot, q, qmax, sid, key);
-        if (key < best) {
-          best = key;
-          id = sid;
+        h = tri_test(m, primIDs, base, cand, q, qmax, sid, key);
+        if (!(key < best)) {
+          key = INFINITY;
+          sid = 0x7fffffff;
+        }
+      }
+      bool owner = gl == 0;
+      if (SEEDED) {
+        const float okey = __shfl_xor_sync(ones << shift, key, 1);
+        const int32_t osid = __shfl_xor_sync(ones << shift, sid, 1);
+        const uint32_t ocand = __shfl_xor_sync(ones << shift, cand, 1);
+        const bool mine = key < okey || (key == okey && (gl & 1 ? sid < osid : sid <= osid));
+        owner = gl < 2 && mine;
+        if (!mine) {
+          key = okey;
+          sid = osid;
+          cand = ocand;
+        }
+      }
+      if (sid != 0x7fffffff) {
+        best = key;
+        id = sid;
+        slot = cand;
+        if (owner) {
           P = h.P;
-          if (gl == 0) ownD = h.d;
+          ownD = h.d;
         }
       }
       reach = tri_reach(best, qmax);
@@ -355,7 +432,7 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
     // take nodes; until a triangle is known nothing can be left out, so a
     // narrow front keeps the stack short on the way down
     const uint32_t w = min(min(id >= 0 || best < 3e38f ? (uint32_t)G : 2u, sp), (uint32_t)CAP - sp);
-    const bool left = busy && sp != 0 && (w == 0 || (!HEAVY && ++steps > TRI_STEP_LIMIT));
+    const bool left = busy && sp != 0 && (w == 0 || (LIMIT && ++steps > LIMIT));
     bool act = busy && gl < w;
     sp -= w;
     StackEntry e{0, 0.f};
@@ -467,6 +544,66 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
   }
 }
 
+// A thread a query, the warps in step, for `rounds` rounds (in a batch, none
+// for warps whose meshes are all too large); what is not answered then goes on
+// a list, with the place of the triangle found so far in outIds.
+__global__ void __launch_bounds__(128) k_tri_near(TriMesh m, const float *__restrict__ queries,
+                                                  const uint32_t *__restrict__ order, uint32_t nq, uint32_t rounds,
+                                                  float maxSqr, int32_t *outIds, float *outD, float *outP,
+                                                  uint32_t *leftList, uint32_t *leftCount)
+{
+  griddep_wait();
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, tt = min(t, nq - 1);
+  const uint32_t qi = order ? __ldg(order + tt) : tt;
+  const float *p = queries + 3ull * qi;
+  const V3 q{__ldg(p), __ldg(p + 1), __ldg(p + 2)};
+  const Node *nodes = m.nodes;
+  const uint32_t *primIDs = m.primIDs;
+  uint32_t base = 0;
+  bool tree = true;
+  if (m.bvhs) {
+    const uint32_t s = seg_find(m.queryOff, m.numSegs, qi);
+    const bq_bvh3f d = m.bvhs[s];
+    if (__all_sync(0xffffffffu, d.numPrims > TRI_NEAR_PRIMS)) rounds = 0;
+    nodes = (const Node *)d.nodes;
+    primIDs = d.primIDs;
+    base = __ldg(m.triOff + s);
+    tree = d.numNodes != 0;
+  }
+  TriNear leaf(m, primIDs, base, q, maxSqr);
+  LocalStack<TRI_NEAR_STACK> st;
+  const bool ok = traverse_warp<TIE_LOWEST, true>(nodes, q.x, q.y, q.z, leaf.cull(), st, leaf, t < nq && tree, rounds);
+  if (t < nq) {
+    if (ok) {
+      outIds[qi] = leaf.id;
+      outD[qi] = leaf.d;
+      if (outP) {
+        outP[3ull * qi] = leaf.P.x;
+        outP[3ull * qi + 1] = leaf.P.y;
+        outP[3ull * qi + 2] = leaf.P.z;
+      }
+    } else {
+      outIds[qi] = leaf.id >= 0 ? (int32_t)leaf.slot : -1;
+    }
+  }
+  list_append(t < nq && !ok, qi, leftList, leftCount);
+}
+
+// the queries of that list, by groups, each `run` next to each other
+__global__ void __launch_bounds__(128, 8) k_tri_left(TriMesh m, const float *__restrict__ queries, uint32_t run,
+                                                     float maxSqr, int32_t *outIds, float *outD, float *outP,
+                                                     const uint32_t *__restrict__ list, const uint32_t *listCount,
+                                                     uint32_t *leftList, uint32_t *leftCount)
+{
+  griddep_wait();
+  __shared__ TriGroupShared<TRI_GROUP, TRI_GROUP_STACK> sh[128 / TRI_GROUP];
+  const uint32_t g = threadIdx.x / TRI_GROUP, nq = *listCount;
+  const uint64_t at = ((uint64_t)blockIdx.x * (128 / TRI_GROUP) + g) * run;
+  const uint32_t b = (uint32_t)min(at, (uint64_t)nq), e = (uint32_t)min(at + run, (uint64_t)nq);
+  tri_group<TRI_GROUP, TRI_GROUP_STACK, true, TRI_STEP_LIMIT>(m, queries, list, b, e, 1, maxSqr, outIds, outD, outP,
+                                                              leftList, leftCount, sh[g]);
+}
+
 // each group answers `run` queries next to each other in the visiting order
 __global__ void __launch_bounds__(128, 8) k_tri_group(TriMesh m, const float *__restrict__ queries,
                                                    const uint32_t *__restrict__ order, uint32_t nq, uint32_t run,
@@ -478,8 +615,8 @@ __global__ void __launch_bounds__(128, 8) k_tri_group(TriMesh m, const float *__
   const uint32_t g = threadIdx.x / TRI_GROUP;
   const uint64_t at = ((uint64_t)blockIdx.x * (128 / TRI_GROUP) + g) * run;
   const uint32_t b = (uint32_t)min(at, (uint64_t)nq), e = (uint32_t)min(at + run, (uint64_t)nq);
-  tri_group<TRI_GROUP, TRI_GROUP_STACK, false>(m, queries, order, b, e, 1, maxSqr, outIds, outD, outP, leftList,
-                                               leftCount, sh[g]);
+  tri_group<TRI_GROUP, TRI_GROUP_STACK, false, TRI_STEP_LIMIT>(m, queries, order, b, e, 1, maxSqr, outIds, outD, outP,
+                                                               leftList, leftCount, sh[g]);
 }
 
 __global__ void __launch_bounds__(128) k_tri_heavy(TriMesh m, const float *__restrict__ queries, float maxSqr,
@@ -490,7 +627,7 @@ __global__ void __launch_bounds__(128) k_tri_heavy(TriMesh m, const float *__res
   griddep_wait();
   __shared__ TriGroupShared<32, TRI_HEAVY_STACK> sh[4];
   const uint32_t warp = threadIdx.x >> 5;
-  tri_group<32, TRI_HEAVY_STACK, true>(m, queries, list, blockIdx.x * 4 + warp, *listCount, gridDim.x * 4, maxSqr,
+  tri_group<32, TRI_HEAVY_STACK, true, 0>(m, queries, list, blockIdx.x * 4 + warp, *listCount, gridDim.x * 4, maxSqr,
                                        outIds, outD, outP, leftList, leftCount, sh[warp]);
 }
 
@@ -513,14 +650,24 @@ __global__ void k_tri_pack(const uint32_t *__restrict__ primIDs, uint32_t numPri
   packed[3ull * j + 2] = make_float4(c.x, c.y, c.z, 0.f);
 }
 
-// the two launches; queries that neither finished are on ovfList.  heavy: a
-// list of nq words, count: two words, zeroed
-inline void launch_tri_group(const TriMesh &m, const float *queries, const uint32_t *order, uint32_t nq, float maxSqr,
-                             int32_t *ids, float *d, float *P, uint32_t *heavy, uint32_t *heavyCount,
-                             uint32_t *ovfList, uint32_t *ovfCount, cudaStream_t s)
+// The launches; queries that none finished are on ovfList.  numPrims: of the
+// tree (0 for a batch: k_tri_near looks at each).  heavy: a list of nq words;
+// the counts are zeroed
+inline void launch_tri_group(const TriMesh &m, uint32_t numPrims, const float *queries, const uint32_t *order, uint32_t nq, float maxSqr,
+                             int32_t *ids, float *d, float *P, uint32_t *heavy, uint32_t *ovfList, uint32_t *ovfCount,
+                             uint32_t *heavyCount, uint32_t *nearCount, cudaStream_t s)
 {
   const uint32_t run = tri_run(nq);
-  {
+  if (nq >= TRI_NEAR_MIN && numPrims <= TRI_NEAR_PRIMS) {
+    {
+      ProfScope ps("tri.near", s);
+      launch_pdl(k_tri_near, dim3(div_up(nq, 128)), dim3(128), 0, s, m, queries, order, nq,
+                 tri_near_rounds(nq), maxSqr, ids, d, P, ovfList, nearCount);
+    }
+    ProfScope ps("tri.group", s);
+    launch_pdl(k_tri_left, dim3(div_up((uint64_t)div_up(nq, run) * TRI_GROUP, 128)), dim3(128), 0, s, m, queries, run,
+               maxSqr, ids, d, P, (const uint32_t *)ovfList, (const uint32_t *)nearCount, heavy, heavyCount);
+  } else {
     ProfScope ps("tri.group", s);
     launch_pdl(k_tri_group, dim3(div_up((uint64_t)div_up(nq, run) * TRI_GROUP, 128)), dim3(128), 0, s, m, queries,
                order, nq, run, maxSqr, ids, d, P, heavy, heavyCount);

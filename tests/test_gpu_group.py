@@ -161,6 +161,24 @@ def test_triangle_slivers_do_not_depend_on_batch_or_tree(bq):
     assert _same(bq.triangles.findClosest(sah, tt, tv, tq), many), "another tree"
 
 
+# the smallest batch a thread a query goes first in, and the next number of rounds; the largest tree and the one after
+@pytest.mark.parametrize("nq", [65535, 65536, 262143, 262144 + 33])
+@pytest.mark.parametrize("n", [1, 1280, 131072, 131073])
+def test_triangle_threads_before_groups(bq, n, nq):
+    """Answered by threads, by groups after them, or by groups alone: the same."""
+    tv, tt = _mesh(7 if n > 1280 else 3, n)
+    g = np.random.default_rng(n)
+    qs = W.uniform_points(nq, 4, -1.5, 1.5)
+    c = tv.cpu().numpy()[tt.cpu().numpy()[g.integers(0, n, nq // 2)]].mean(1)
+    qs[::2][:nq // 2] = c + 0.01 * g.standard_normal(c.shape)  # half of them near the surface
+    qs[7::501] = np.nan
+    tq, bvh = _cuda(qs), bq.cuda.radixBuilder(bq.triangles.boxes(tt, tv))
+    for r in (float("inf"), 0.01):
+        many = bq.triangles.findClosest(bvh, tt, tv, tq, maxSqrDist=r)
+        few = [torch.cat(x) for x in zip(*[bq.triangles.findClosest(bvh, tt, tv, q, maxSqrDist=r) for q in tq.split(30_000)])]
+        assert _same(few, many), f"radius {r}"
+
+
 def test_triangle_groups_heavy_queries(bq):
     """Queries around the middle of a sphere of equal radius visit most of its
     tree and go to the second launch; NaN and infinite ones find nothing."""
