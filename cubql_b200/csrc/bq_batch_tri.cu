@@ -212,27 +212,43 @@ int batched_tri_closest(const bq_bvh3f *bvhs, const uint32_t *triOff, const int3
   uint32_t *err = errOut ? errOut : ctl + 1;
   const int b = c.blockSize;
   if (c.tieMode == BQ_TIES_LOWEST_ID) {
+    // The order and the list of heavy queries save time only: without room for
+    // them the queries are taken as given, and each by a thread.
     uint32_t *heavy = nullptr;
     const uint32_t *order = nullptr;
-    BQ_TRY(tmp.get(&heavy, nq));
     int segBits = 0;
     while (segBits < 32 && (1ull << segBits) < numSegs) segBits++;
     // with few queries a mesh, order within a mesh saves less than it costs
     // (5,000 meshes of 320 triangles, 20 queries each: 0.366 and 0.296 ms)
     if (c.reorder && nq >= TRI_ORDER_MIN && nq / 256 >= numSegs) {
-      uint32_t *keys[2], *idx[2];
-      BQ_TRY(tmp.get(&keys[0], nq));
-      BQ_TRY(tmp.get(&keys[1], nq));
-      BQ_TRY(tmp.get(&idx[0], nq));
-      BQ_TRY(tmp.get(&idx[1], nq));
-      ProfScope ps("batch.query_keys", al.s);
-      launch_pdl(k_btri_keys, dim3(div_up(nq, 256)), dim3(256), 0, al.s, bvhs, queries, nq, qoff, numSegs, segBits,
-                 keys[0], idx[0]);
-      int sel = 0;
-      // order only: 24 bits (3 passes) while they leave the curve at least 16
-      BQ_TRY(onesweep_sort_u32(keys, idx, nq, nullptr, segBits <= 8 ? 8 - std::max(2 - segBits, 0) : 0,
-                               std::min(32, 30 + segBits), nullptr, &sel, err, al));
-      order = idx[sel];
+      const int kept = tmp.n;
+      const int status = [&]() -> int {
+        uint32_t *keys[2], *idx[2];
+        BQ_TRY(tmp.get(&keys[0], nq));
+        BQ_TRY(tmp.get(&keys[1], nq));
+        BQ_TRY(tmp.get(&idx[0], nq));
+        BQ_TRY(tmp.get(&idx[1], nq));
+        ProfScope ps("batch.query_keys", al.s);
+        launch_pdl(k_btri_keys, dim3(div_up(nq, 256)), dim3(256), 0, al.s, bvhs, queries, nq, qoff, numSegs, segBits,
+                   keys[0], idx[0]);
+        int sel = 0;
+        // order only: 24 bits (3 passes) while they leave the curve at least 16
+        BQ_TRY(onesweep_sort_u32(keys, idx, nq, nullptr, segBits <= 8 ? 8 - std::max(2 - segBits, 0) : 0,
+                                 std::min(32, 30 + segBits), nullptr, &sel, err, al));
+        order = idx[sel];
+        heavy = keys[sel];  // the sorted keys are of no further use
+        return BQ_OK;
+      }();
+      if (status == BQ_ERR_ALLOC) {
+        tmp.release(kept);
+        cudaGetLastError();
+      } else {
+        BQ_TRY(status);
+      }
+    }
+    if (!heavy && tmp.get(&heavy, nq) != BQ_OK) {
+      heavy = nullptr;
+      cudaGetLastError();
     }
     const TriMesh m{nullptr, nullptr, bvhs, triOff, qoff, numSegs, nullptr, tris, verts};
     launch_tri_group(m, 0, queries, order, nq, maxSqr, ids, d, P, heavy, ovfList, ctl, ctl + 2, ctl + 3, al.s);

@@ -73,7 +73,7 @@ struct Carver {
 // RAII list of temporaries freed (stream-ordered) at scope exit
 struct TempSet {
   Alloc &al;
-  void *ptrs[32];
+  void *ptrs[32] = {};
   int n = 0;
   explicit TempSet(Alloc &a) : al(a) {}
   template <typename T>
@@ -83,10 +83,12 @@ struct TempSet {
     if (s == BQ_OK) ptrs[n++] = (void *)*p;
     return s;
   }
-  ~TempSet()
+  // gives back all but the first `keep`
+  void release(int keep)
   {
-    for (int i = n - 1; i >= 0; i--) al.scratch_free(ptrs[i]);
+    while (n > keep) al.scratch_free(ptrs[--n]);
   }
+  ~TempSet() { release(0); }
 };
 
 // ------------------------------------------------------------------

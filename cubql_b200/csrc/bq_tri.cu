@@ -284,7 +284,7 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
     return BQ_OK;
   }
   TempSet tmp(al);
-  uint32_t *ovfList = nullptr, *ovfCount = nullptr, *order = nullptr;
+  uint32_t *ovfList = nullptr, *ovfCount = nullptr, *order = nullptr, *heavy = nullptr;
   StackEntry *deep = nullptr;
   BQ_TRY(tmp.get(&ovfList, nq));
   BQ_TRY(tmp.get(&ovfCount, 4));  // overflow count, error word, heavy count, count left by the first launch
@@ -302,6 +302,7 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
     int sel = 0;
     BQ_TRY(onesweep_sort_u32(keys, idx, nq, nullptr, 6, 30, nullptr, &sel, err, al));  // order only: top 24 bits
     order = idx[sel];
+    heavy = keys[sel];  // the sorted keys are of no further use
   }
   const int b = c.blockSize;
 #define BQ_TRI_LAUNCH(TIE, ST)                                                                                     \
@@ -316,9 +317,11 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
     else if (c.stackDepth == 64) { BQ_TRI_LAUNCH(TIE_REFERENCE, 64); }
     else { BQ_TRI_LAUNCH(TIE_REFERENCE, 128); }
   } else {
-    uint32_t *heavy = nullptr;
     float4 *packed = nullptr;
-    BQ_TRY(tmp.get(&heavy, nq));
+    if (!heavy && tmp.get(&heavy, nq) != BQ_OK) {
+      heavy = nullptr;
+      cudaGetLastError();
+    }
     // a query tests some twenty triangles: the copy pays from about a
     // twentieth as many queries as triangles
     if ((uint64_t)nq * 16 >= bvh->numPrims) {

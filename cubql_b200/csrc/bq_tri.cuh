@@ -544,9 +544,11 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
   }
 }
 
-// A thread a query, the warps in step, for `rounds` rounds (in a batch, none
-// for warps whose meshes are all too large); what is not answered then goes on
-// a list, with the place of the triangle found so far in outIds.
+// A thread a query, the warps in step, for `rounds` rounds (TRI_ALL: to the
+// end; in a batch, none for warps whose meshes are all too large); what is not
+// answered then goes on a list, with the place of the triangle found so far in
+// outIds.
+constexpr uint32_t TRI_ALL = 0xffffffffu;
 __global__ void __launch_bounds__(128) k_tri_near(TriMesh m, const float *__restrict__ queries,
                                                   const uint32_t *__restrict__ order, uint32_t nq, uint32_t rounds,
                                                   float maxSqr, int32_t *outIds, float *outD, float *outP,
@@ -564,7 +566,7 @@ __global__ void __launch_bounds__(128) k_tri_near(TriMesh m, const float *__rest
   if (m.bvhs) {
     const uint32_t s = seg_find(m.queryOff, m.numSegs, qi);
     const bq_bvh3f d = m.bvhs[s];
-    if (__all_sync(0xffffffffu, d.numPrims > TRI_NEAR_PRIMS)) rounds = 0;
+    if (__all_sync(0xffffffffu, d.numPrims > TRI_NEAR_PRIMS) && rounds != TRI_ALL) rounds = 0;
     nodes = (const Node *)d.nodes;
     primIDs = d.primIDs;
     base = __ldg(m.triOff + s);
@@ -651,13 +653,20 @@ __global__ void k_tri_pack(const uint32_t *__restrict__ primIDs, uint32_t numPri
 }
 
 // The launches; queries that none finished are on ovfList.  numPrims: of the
-// tree (0 for a batch: k_tri_near looks at each).  heavy: a list of nq words;
-// the counts are zeroed
+// tree (0 for a batch: k_tri_near looks at each).  heavy: a list of nq words, or
+// null when there is no room for one: each query is then answered by a thread.
+// The counts are zeroed.
 inline void launch_tri_group(const TriMesh &m, uint32_t numPrims, const float *queries, const uint32_t *order, uint32_t nq, float maxSqr,
                              int32_t *ids, float *d, float *P, uint32_t *heavy, uint32_t *ovfList, uint32_t *ovfCount,
                              uint32_t *heavyCount, uint32_t *nearCount, cudaStream_t s)
 {
   const uint32_t run = tri_run(nq);
+  if (!heavy) {
+    ProfScope ps("tri.near", s);
+    launch_pdl(k_tri_near, dim3(div_up(nq, 128)), dim3(128), 0, s, m, queries, order, nq, TRI_ALL, maxSqr, ids, d, P,
+               ovfList, ovfCount);
+    return;
+  }
   if (nq >= TRI_NEAR_MIN && numPrims <= TRI_NEAR_PRIMS) {
     {
       ProfScope ps("tri.near", s);

@@ -179,6 +179,45 @@ def test_triangle_threads_before_groups(bq, n, nq):
         assert _same(few, many), f"radius {r}"
 
 
+def _limited_allocator(bq, limit):
+    """Blocks from torch, `limit` bytes (a list of one number) of them at a time."""
+    class Limited(bq.TorchAllocator):
+        def _malloc(self, ctx, out, size, stream):
+            if sum(t.numel() for t in self.live.values()) + size > limit[0]:
+                return 1
+            return super()._malloc(ctx, out, size, stream)
+
+    a = Limited()
+    a.c.scratchFromPool = 0
+    return a
+
+
+def test_triangle_queries_need_no_more_scratch_than_a_thread_a_query(bq):
+    """With room for the overflow list and the deep stacks alone (and, for one tree, the sort), the answers are the
+    same as with room for the order, the list of heavy queries and the copy of the corners."""
+    tv, tt = _mesh(4)
+    boxes = bq.triangles.boxes(tt, tv)
+    tq = _cuda(W.uniform_points(100_000, 4, -1.5, 1.5))
+    least = 4 * len(tq) + 2048 * 1024 * 8 + 4096
+    off, qoff = _cuda(np.array([0, 2000, 2000, len(tt)])), _cuda(np.array([0, 40_000, 40_100, len(tq)]))
+    batch = bq.Batch(boxes, off)
+    want = bq.batched_tri_closest(batch, tt, tv, tq, qoff)
+    limit = [1 << 40]
+    alloc = _limited_allocator(bq, limit)
+    for extra in (0, 4, 12, 16, 20):  # bytes a query
+        limit[0] = least + extra * len(tq)
+        assert _same(bq.batched_tri_closest(batch, tt, tv, tq, qoff, allocator=alloc), want), extra
+    limit[0] = 1 << 40
+    bvh = bq.cuda.radixBuilder(boxes, None, alloc)
+    want = bq.triangles.findClosest(bvh, tt, tv, tq)
+    tree = sum(t.numel() for t in alloc.live.values())
+    for extra, reorder in ((0, 0), (4, 0), (24, 1)):
+        limit[0] = tree + least + extra * len(tq)
+        got = bq.triangles.findClosest(bvh, tt, tv, tq, qcfg=bq.query_config(reorder=reorder))
+        assert _same(got, want), (extra, reorder)
+    bvh.free()
+
+
 def test_triangle_groups_heavy_queries(bq):
     """Queries around the middle of a sphere of equal radius visit most of its
     tree and go to the second launch; NaN and infinite ones find nothing."""
