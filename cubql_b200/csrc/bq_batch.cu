@@ -390,10 +390,12 @@ __global__ void __launch_bounds__(128, GroupShape<K>::BLOCKS)
     if (d.numNodes == 0) continue;  // no prims: the empty list is the answer
     const Node *nodes = (const Node *)d.nodes;
     bool in = false, done = false;
-    if (group_pays(__ldg(qoff + s0 + 1) - __ldg(qoff + s0), d.numPrims)) {
+    const uint32_t cloudQueries = __ldg(qoff + s0 + 1) - __ldg(qoff + s0);
+    if (cloudQueries >= 16 && group_pays(cloudQueries, d.numPrims, k) &&
+        group_radius_pays(nodes, d.numPrims, maxSqr, k)) {
       in = mine && group_can_search(nodes, qx, qy, qz);
-      done = group_search<K>(nodes, d.primIDs, points + 3ull * __ldg(poff + s0), in, qx, qy, qz, maxSqr, list,
-                             sh[threadIdx.x >> 5]);
+      done = group_search<K>(nodes, d.primIDs, points + 3ull * __ldg(poff + s0), in, qx, qy, qz, maxSqr,
+                             cloudQueries, d.numPrims, list, sh[threadIdx.x >> 5]);
     }
     if (mine && !(done && in)) {
       left = true;
@@ -474,8 +476,12 @@ __global__ void __launch_bounds__(128) k_seg_knn(const bq_bvh3f *__restrict__ bv
       leaf.maxSqr = maxSqr;
       leaf.list.init(k);
       LocalStack<STACK> st;
-      const bool ok = traverse_warp<TIE>((const Node *)d.nodes, leaf.qx, leaf.qy, leaf.qz, maxSqr, st, leaf,
-                                         alive && d.numNodes != 0);
+      bool ok = true;
+      if constexpr (K > 4)
+        ok = traverse_warp<TIE>((const Node *)d.nodes, leaf.qx, leaf.qy, leaf.qz, maxSqr, st, leaf,
+                                alive && d.numNodes != 0);
+      else if (alive && d.numNodes != 0)  // short lists are cheap to insert into: leaves are taken at once
+        ok = traverse<TIE>((const Node *)d.nodes, leaf.qx, leaf.qy, leaf.qz, maxSqr, st, leaf);
       if (!alive) continue;
       if (!ok) {
         ovfList[atomicAdd(ovfCount, 1u)] = t;
@@ -538,14 +544,16 @@ int launch_seg_knn(const bq_bvh3f *bvhs, const uint32_t *poff, const float *poin
                    int block, int chunk, uint32_t *workCtr, int32_t *ids, float *d, int32_t *nf, uint32_t *ovfList,
                    uint32_t *ovfCount, StackEntry *deep, uint32_t *leftList, uint32_t *err, cudaStream_t s)
 {
-  if (TIE == TIE_LOWEST && K <= 32 && order) {
-    ProfScope ps("batch.knn", s);
-    constexpr int KK = K <= 32 ? K : 32;
-    launch_pdl(k_seg_knn_warp<KK>, dim3(div_up(nq, block)), dim3(block), 0, s, bvhs, poff, points, queries, qoff,
-               skeys, order, nq, k, maxSqr, ids, d, nf, leftList, workCtr);
-    launch_pdl(k_seg_knn_left<KK, STACK>, dim3(std::min(div_up(nq, 128), 8 * num_sms())), dim3(128), 0, s, bvhs, poff,
-               points, queries, skeys, order, (const uint32_t *)leftList, (const uint32_t *)workCtr, k, maxSqr, ids, d,
-               nf, ovfList, ovfCount);
+  if (TIE == TIE_LOWEST && K > 4 && K <= 32 && order) {
+    constexpr int KK = K > 4 && K <= 32 ? K : 32;
+    {
+      ProfScope ps("batch.knn_shared", s);
+      launch_pdl(k_seg_knn_warp<KK>, dim3(div_up(nq, block)), dim3(block), 0, s, bvhs, poff, points, queries, qoff,
+                 skeys, order, nq, k, maxSqr, ids, d, nf, leftList, workCtr);
+    }
+    ProfScope ps("batch.knn_left", s);
+    launch_pdl(k_seg_knn_left<KK, STACK>, dim3(knn_left_blocks(nq)), dim3(128), 0, s, bvhs, poff, points, queries, skeys,
+               order, (const uint32_t *)leftList, (const uint32_t *)workCtr, k, maxSqr, ids, d, nf, ovfList, ovfCount);
   } else {
     int perSm = 0;
     BQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_seg_knn<K, TIE, STACK>, block, 0));

@@ -102,7 +102,8 @@ __device__ __forceinline__ float warp_max_f(float x) { return dec_f(__reduce_max
 template <int K>
 __device__ __forceinline__ bool group_search(const Node *__restrict__ nodes, const uint32_t *__restrict__ primIDs,
                                              const float *__restrict__ points, bool in, float qx, float qy, float qz,
-                                             float maxSqr, KnnList<K, TIE_LOWEST> &list, GroupShared<K> &sh)
+                                             float maxSqr, uint32_t numQueries, uint32_t numPrims,
+                                             KnnList<K, TIE_LOWEST> &list, GroupShared<K> &sh)
 {
   constexpr int P = GroupShape<K>::P, C = GroupShape<K>::C;
   const uint32_t lane = threadIdx.x & 31;
@@ -112,6 +113,18 @@ __device__ __forceinline__ bool group_search(const Node *__restrict__ nodes, con
               lz = warp_min_f(in ? qz : INFINITY);
   const float hx = warp_max_f(in ? qx : -INFINITY), hy = warp_max_f(in ? qy : -INFINITY),
               hz = warp_max_f(in ? qz : -INFINITY);
+  const float diag2 = (hx - lx) * (hx - lx) + (hy - ly) * (hy - ly) + (hz - lz) * (hz - lz);
+  {
+    // Queries far from their neighbours on the curve, as those outside the
+    // root's box are (the curve ends there): spread over 1,024 times the
+    // space of 32 queries.  1M queries of which 1 in 27 is inside, 2M points,
+    // k = 16: 4.3 ms without this, 3.4 with it, 3.6 one thread per query.
+    const Node root = ldg_node(nodes);
+    const float ext = fmaxf(fmaxf(root.a.w - root.a.x, root.b.x - root.a.y), root.b.y - root.a.z);
+    if (diag2 * sqrtf(diag2) * (float)numQueries > 32.f * 1024.f * ext * ext * ext) return false;
+  }
+  // (dense queries: the box is small against the prims' spacing)
+  const float far = (uint64_t)numQueries < 4ull * numPrims ? 4.f * diag2 : INFINITY;
   // a prim is wanted at up to `mine`: below the radius, and no farther than
   // the k-th best (at the same distance its id decides)
   const float limit = maxSqr > 0.f ? __uint_as_float(__float_as_uint(maxSqr) - 1) : -1.f;
@@ -199,14 +212,21 @@ __device__ __forceinline__ bool group_search(const Node *__restrict__ nodes, con
       __syncwarp();
     }
     if (sp == 0) break;  // the queue is empty too
-    // The queries are too far apart for one search when fewer than one lane
-    // wanted each prim that was tested, or far more prims were tested than a
-    // compact warp needs and not nearly every lane wanted them (copies of one
-    // point are wanted by all).  Queries far from the prims they look for are
-    // the case: without the second limit a warp tests thousands of prims.
-    // 2 clouds, one of them clusters: 1.22 ms with both, 2.76 with the first
-    // alone, 1.42 one thread per query; 512 clouds 69.8, 75.9, 83.8.
-    if (tested > 512 + 16 * K && wanted < (tested > 512 + 64 * K ? 8 : 1) * tested) return false;
+    // The queries have too little in common for one search when their prims
+    // are farther away than twice the size of their box (the shell between
+    // the nearest and the farthest lane's reach holds thousands of prims),
+    // when fewer than one lane wanted each prim that was tested, or when far
+    // more prims were tested than a compact warp needs and not nearly every
+    // lane wanted them (copies of one point are wanted by all).  500,000
+    // queries in a cube, 1M points on a plane in it, k = 32: 7.2 ms without
+    // the first, 3.8 with it, 4.4 one thread per query before; 300,000 points
+    // on a line, k = 16: 37, 10 and 7.6 (the last limit: 13 without it).  The
+    // limits on prims, 2 clouds, one of them clusters: 1.22 ms with 512 + 16 K
+    // and 512 + 64 K, 2.76 with the first alone, 1.42 one thread per query.
+    if (bounded && reach > far) return false;
+    if (tested > 512 + 16 * K &&
+        wanted < (tested > 2048 + 128 * K ? 16 : tested > 512 + 64 * K ? 8 : 1) * tested)
+      return false;
     // Until k prims are known to every lane nothing can be left out: a
     // narrow front then keeps the stack short on the way down.
     const uint32_t w = min(min(bounded ? 16u : 4u, sp), (uint32_t)GROUP_STACK - sp);
@@ -246,15 +266,41 @@ __device__ __forceinline__ bool group_search(const Node *__restrict__ nodes, con
 }
 
 // Whether the queries are dense enough among the prims for a warp's 32 to
-// share a search (a warp whose queries are not gives up by itself).  Below
-// this the box of 32 queries holds hundreds of prims that no lane wants:
-// 200,000 queries over 3M points, k = 16, take 1.95 ms shared and 1.0 ms one
-// thread each; 3,000 over 5M 4.3 and 0.32 ms; 1M over 2M, k = 32, 3.7 and
-// 10.5 ms.
-__host__ __device__ inline bool group_pays(uint32_t numQueries, uint32_t numPrims)
+// share a search.  Fewer queries have wide boxes that hold many prims no lane
+// wants, and short lists are found sooner by a thread.  Uniform points, ms
+// shared and a thread a query (k <= 5 plain, above in step), by queries a
+// prim.  2M points: k = 1 at 1 1.27 and 1.01, at 4 2.81 and 3.26; k = 4 at 1
+// 1.51 and 1.84 (but clustered data lose), at 2 2.12 and 3.23; k = 8 at 1/4
+// 1.06 and 0.98, at 1 2.00 and 3.01; k = 16 at 1/4 1.82 and 1.58, at 1 3.55
+// and 5.08; k = 32 at 1/4 2.88 and 3.21, at 1/2 3.78 and 5.77.  200,000
+// points: k = 16 at 1/2 0.52 and 0.41, at 1 0.48 and 0.66.  20,000: k = 8 at 1
+// 0.22 and 0.20, at 2 0.16 and 0.21; k = 16 at 1/2 0.37 and 0.24 (too few
+// warps to hide the steps).
+__host__ __device__ inline bool group_pays(uint32_t numQueries, uint32_t numPrims, int k)
 {
-  return (uint64_t)numQueries * 8 >= numPrims;
+  const uint64_t q = numQueries, p = numPrims;
+  if (k == 1) return q >= 4 * p && p >= 32768;
+  if (k <= 4) return q >= 2 * p && p >= 1024;
+  if (k <= 16) return (q >= p || (2 * q >= p && q >= (1u << 19))) && p >= 32;
+  return 2 * q >= p && p >= 32;
 }
+
+// Whether a ball of a finite radius can be expected to hold half the k prims
+// that are looked for (were they spread evenly over the root's box).
+__device__ __forceinline__ bool group_radius_pays(const Node *nodes, uint32_t numPrims, float maxSqr, int k)
+{
+  if (!(maxSqr < INFINITY)) return true;
+  const Node n = ldg_node(nodes);
+  const float r = sqrtf(fmaxf(maxSqr, 0.f));
+  const float vx = fmaxf(n.a.w - n.a.x, r), vy = fmaxf(n.b.x - n.a.y, r), vz = fmaxf(n.b.y - n.a.z, r);
+  return 8.f * r / vx * r / vy * r / vz * (float)numPrims >= (float)k;
+}
+
+// Blocks of 128 threads for the queries that the shared search has left: one
+// for every 128 queries of the call, though most find nothing, as those left
+// take very different times.  512 clouds: 62 ms with 8 an SM that go through
+// the list, 59 with 64, 57.5 so.
+inline int knn_left_blocks(uint32_t nq) { return div_up(nq, 128); }
 
 // whether a query can take part: it is finite and its distance to the tree
 // does not overflow (such a query would keep the reach infinite)

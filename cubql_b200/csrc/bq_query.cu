@@ -45,6 +45,11 @@ constexpr int KNN_SMEM_STACK = 0;
 // from the start (k = 32, 1,001: 0.195 and 0.259).
 constexpr uint32_t CP_ORDER_MIN = 1u << 17;
 inline uint32_t knn_order_min(int k) { return k <= 8 ? 4096 : 2; }
+// Longest lists whose searches, a thread each, do not walk in step: inserting
+// into them costs little, so leaves are better taken at once (2M points and
+// queries, plain and in step, ms: k = 1 1.01 and 1.26, 4 1.84 and 1.99, 5 2.31
+// and 2.47, 8 3.09 and 3.01, 16 6.75 and 5.08).
+constexpr int KNN_PLAIN_MAX = 5;
 
 // rootBox: lower xyz, upper xyz (the first 24 bytes of a binary root node)
 template <bool HILBERT>
@@ -193,8 +198,8 @@ __device__ __forceinline__ bool run_knn(bool alive, const Node *nodes, const uin
 // on a list, with what is known of their k-th best distance in outD
 template <int K>
 __global__ void __launch_bounds__(128, GroupShape<K>::BLOCKS)
-    k_knn_warp(const Node *__restrict__ nodes, const uint32_t *__restrict__ primIDs, const float *__restrict__ points,
-               const float *__restrict__ queries, const uint32_t *__restrict__ order, uint32_t nq, int k, float maxSqr,
+    k_knn_warp(const Node *__restrict__ nodes, uint32_t numPrims, const uint32_t *__restrict__ primIDs,
+               const float *__restrict__ points, const float *__restrict__ queries, const uint32_t *__restrict__ order, uint32_t nq, int k, float maxSqr,
                int32_t *__restrict__ outIds, float *__restrict__ outD, int32_t *__restrict__ numFound,
                uint32_t *__restrict__ leftList, uint32_t *leftCount)
 {
@@ -208,7 +213,10 @@ __global__ void __launch_bounds__(128, GroupShape<K>::BLOCKS)
   const bool in = alive && group_can_search(nodes, qx, qy, qz);
   KnnList<K, TIE_LOWEST> list;
   list.init(k);
-  const bool done = group_search<K>(nodes, primIDs, points, in, qx, qy, qz, maxSqr, list, sh[threadIdx.x >> 5]) && in;
+  const bool done = group_radius_pays(nodes, numPrims, maxSqr, k) &&
+                    group_search<K>(nodes, primIDs, points, in, qx, qy, qz, maxSqr, nq, numPrims, list,
+                                    sh[threadIdx.x >> 5]) &&
+                    in;
   if (alive && done) write_knn(list, qi, k, outIds, outD, numFound);
   const bool left = alive && !done;
   if (left) outD[(size_t)qi * k] = in ? fminf(maxSqr, list.worst()) : maxSqr;
@@ -236,7 +244,7 @@ __global__ void __launch_bounds__(128) k_knn_left(const Node *__restrict__ nodes
   }
 }
 
-template <int K, int TIE, int STACK>
+template <int K, int TIE, int STACK, bool STEP>
 __global__ void __launch_bounds__(128) k_knn(const Node *__restrict__ nodes, const uint32_t *__restrict__ primIDs,
                                              const float *__restrict__ points, const float *__restrict__ queries,
                                              const uint32_t *__restrict__ order, uint32_t nq, int k, float maxSqr,
@@ -246,11 +254,12 @@ __global__ void __launch_bounds__(128) k_knn(const Node *__restrict__ nodes, con
 {
   griddep_wait();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool alive = t < nq;  // no early return: the warp walks in step
+  const bool alive = t < nq;
+  if (!STEP && !alive) return;  // in step the whole warp stays
   const uint32_t qi = order ? __ldg(order + min(t, nq - 1)) : min(t, nq - 1);
   extern __shared__ StackEntry sStack[];
   HybridStack<KNN_SMEM_STACK, STACK> st(sStack);
-  if (!run_knn<K, TIE, true>(alive, nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD, numFound))
+  if (!run_knn<K, TIE, STEP>(alive, nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD, numFound))
     ovfList[atomicAdd(ovfCount, 1u)] = qi;
 }
 
@@ -462,23 +471,25 @@ void launch_knn(const bq_bvh3f *bvh, const float *points, const float *queries, 
                 int block, int32_t *ids, float *d, int32_t *nf, QueryScratch &qs, cudaStream_t s)
 {
   const Node *nodes = (const Node *)bvh->nodes;
-  {
-    ProfScope ps("query.knn", s);
-    // The shared search needs an answer that does not depend on the visiting
-    // order, queries sorted along the curve and lists that fit its registers
-    // (k > 32 would need 246 a thread).
-    if (TIE == TIE_LOWEST && K <= 32 && qs.order && group_pays(nq, bvh->numPrims)) {
-      constexpr int KK = K <= 32 ? K : 32;
-      launch_pdl(k_knn_warp<KK>, dim3(div_up(nq, block)), dim3(block), 0, s, nodes, bvh->primIDs, points, queries,
-                 qs.order, nq, k, maxSqr, ids, d, nf, qs.leftList, qs.ovfCount + 2);
-      launch_pdl(k_knn_left<KK, STACK>, dim3(std::min(div_up(nq, 128), 8 * num_sms())), dim3(128), 0, s, nodes,
-                 bvh->primIDs, points, queries, (const uint32_t *)qs.leftList, (const uint32_t *)(qs.ovfCount + 2), k,
-                 maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);
+  // The shared search needs an answer that does not depend on the visiting
+  // order, queries sorted along the curve and lists that fit its registers
+  // (k > 32 would need 246 a thread).
+  if (TIE == TIE_LOWEST && K <= 32 && qs.leftList) {
+    constexpr int KK = K <= 32 ? K : 32;
+    {
+      ProfScope ps("query.knn_shared", s);
+      launch_pdl(k_knn_warp<KK>, dim3(div_up(nq, block)), dim3(block), 0, s, nodes, bvh->numPrims, bvh->primIDs, points,
+                 queries, qs.order, nq, k, maxSqr, ids, d, nf, qs.leftList, qs.ovfCount + 2);
     }
-    else
-      launch_pdl(k_knn<K, TIE, STACK>, dim3(div_up(nq, block)), dim3(block),
-                 KNN_SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries, qs.order, nq, k,
-                 maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);
+    ProfScope ps("query.knn_left", s);
+    launch_pdl(k_knn_left<KK, STACK>, dim3(knn_left_blocks(nq)), dim3(128), 0, s, nodes, bvh->primIDs, points, queries,
+               (const uint32_t *)qs.leftList, (const uint32_t *)(qs.ovfCount + 2), k, maxSqr, ids, d, nf, qs.ovfList,
+               qs.ovfCount);
+  } else {
+    ProfScope ps("query.knn", s);
+    launch_pdl(k > KNN_PLAIN_MAX ? k_knn<K, TIE, STACK, (K > 4)> : k_knn<K, TIE, STACK, (K > 8)>, dim3(div_up(nq, block)),
+               dim3(block), KNN_SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries,
+               qs.order, nq, k, maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);
   }
   ProfScope ps("query.deep", s);
   launch_pdl(k_knn_deep<K, TIE>, dim3(DEEP_THREADS / 128), dim3(128), 0, s, nodes, bvh->primIDs, points, queries, k,
@@ -602,7 +613,7 @@ int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, boo
     const int loBit = nq <= (1u << 21) ? 14 : 6;
     BQ_TRY(onesweep_sort_u32(keys, idx, nq, nullptr, loBit, 30, nullptr, &sel, qs.err, al));
     qs.order = idx[sel];
-    qs.leftList = keys[sel];  // the sorted keys are of no further use
+    if (hilbert) qs.leftList = keys[sel];  // the sorted keys are of no further use
   }
   return BQ_OK;
 }
@@ -687,7 +698,7 @@ int knn(const bq_bvh3f *bvh, const float *points, const float *queries, uint32_t
   // one search for a warp's queries (launch_knn); its order is the curve
   // without jumps
   const bool shared =
-      c.tieMode == BQ_TIES_LOWEST_ID && k <= 32 && c.lanesPerQuery == 1 && group_pays(nq, bvh->numPrims);
+      c.tieMode == BQ_TIES_LOWEST_ID && k <= 32 && c.lanesPerQuery == 1 && group_pays(nq, bvh->numPrims, k);
   BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0 && nq >= knn_order_min(k), shared, tmp, al, qs));
   const int tie = c.tieMode, st = c.stackDepth, b = c.blockSize;
   if (c.lanesPerQuery > 1) {

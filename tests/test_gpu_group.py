@@ -19,60 +19,99 @@ def _same(a, b):
     return all(torch.equal(x, y) for x, y in zip(a, b))
 
 
-# sizes around a warp; radii from none to all; k around the list sizes; leaves of one and of many prims
-@pytest.mark.parametrize("nq", [2, 31, 32, 33, 4097])
-@pytest.mark.parametrize("k", [1, 4, 5, 16, 17, 32])
-@pytest.mark.parametrize("n,leaf", [(1, 1), (3, 1), (40, 8), (20000, 1), (20000, 40)])
-def test_knn_shared_search_equals_one_thread_per_query(bq, nq, k, n, leaf):
+def _phases(bq, call):
+    """(result, names of the phases that ran)"""
+    with bq.profile() as prof:
+        r = call()
+    return r, set(prof.table)
+
+
+def _knn_both_ways(bq, bvh, tp, tq, k, shared, **kw):
+    """The search as it is chosen (and that it is the shared one, or not), and with a thread a query in the given
+    order; they have to be the same."""
+    a, ran = _phases(bq, lambda: bq.points.findKNN(bvh, tp, tq, k, **kw))
+    b, ran0 = _phases(bq, lambda: bq.points.findKNN(bvh, tp, tq, k, qcfg=bq.query_config(reorder=0), **kw))
+    assert "query.knn_shared" not in ran0 and ("query.knn_shared" in ran) == shared, (ran, ran0)
+    assert _same(a, b), (k, kw)
+    return a
+
+
+# batches whose last warp is whole, one query, all but one; radii from none to all; k around the list sizes; leaves of
+# one and of many prims
+@pytest.mark.parametrize("extra", [0, 1, 31, 33])
+@pytest.mark.parametrize("k", [2, 4, 5, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("n,leaf", [(32, 1), (1024, 1), (1024, 40), (3000, 8)])
+def test_knn_shared_search_equals_one_thread_per_query(bq, extra, k, n, leaf):
+    nq = (6016 if k <= 16 else 1504) + extra
     pts, qs = W.uniform_points(n), W.uniform_points(nq, W.SEED_QUERIES, -0.1, 1.1)
     tp, tq = _cuda(pts), _cuda(qs)
     bvh = bq.cuda.radixBuilder(_cuda(boxes_np(pts)), bq.BuildConfig(makeLeafThreshold=leaf))
-    for r in (float("inf"), 0.01, 0.0):
-        a = bq.points.findKNN(bvh, tp, tq, k, maxSqrDist=r)
-        b = bq.points.findKNN(bvh, tp, tq, k, maxSqrDist=r, qcfg=bq.query_config(reorder=0))
-        assert _same(a, b), f"radius {r}"
+    for r in (float("inf"), 0.3, 0.01, 0.0):
+        _knn_both_ways(bq, bvh, tp, tq, k, n >= 1024 or k > 4, maxSqrDist=r)
+    bvh.free()
+
+
+# either side of each line that decides between the shared search and a thread a query
+@pytest.mark.parametrize("n,nq,k,shared", [
+    (32768, 131072, 1, True), (32768, 131071, 1, False), (32767, 140000, 1, False),
+    (5000, 10000, 4, True), (5000, 9999, 4, False), (1023, 9999, 4, False),
+    (6000, 6000, 5, True), (6000, 5999, 16, False), (1 << 20, 1 << 19, 9, True), (1 << 20, (1 << 19) - 1, 9, False),
+    (32, 5000, 16, True), (31, 5000, 16, False), (4000, 2000, 17, True), (4000, 1999, 32, False),
+    (2000, 4096, 8, True), (2000, 4095, 8, False), (5000, 9000, 33, False)])
+def test_knn_where_the_shared_search_begins(bq, n, nq, k, shared):
+    pts = W.uniform_points(n)
+    bvh = bq.cuda.radixBuilder(_cuda(boxes_np(pts)))
+    _knn_both_ways(bq, bvh, _cuda(pts), _cuda(W.uniform_points(nq, 3)), k, shared)
     bvh.free()
 
 
 def test_knn_shared_search_on_duplicates_and_clusters(bq):
-    """Copies of points (ids decide) and tight clusters that uniform queries
-    are far from (their warps give the shared search up)."""
+    """Copies of points (ids decide); tight clusters, planes and lines that
+    the queries are far from, and queries far outside: their warps give the
+    shared search up."""
     rng = np.random.default_rng(3)
+    u = W.uniform_points(20000, 9)
     dup = np.repeat(W.uniform_points(300), 40, axis=0)
-    clu = (W.uniform_points(8, 5)[rng.integers(0, 8, 30000)] + 0.002 * rng.standard_normal((30000, 3))).astype(np.float32)
-    for pts, qs in ((dup, np.concatenate([dup[::7], W.uniform_points(3000, 9)])), (clu, W.uniform_points(20000, 9))):
+    clu = (W.uniform_points(8, 5)[rng.integers(0, 8, 20000)] + 0.002 * rng.standard_normal((20000, 3))).astype(np.float32)
+    for pts, qs in ((dup, np.concatenate([dup[::2], W.uniform_points(9000, 9)])), (clu, u),
+                    (u * np.float32([1, 1, 0]), u), (u * np.float32([1, 0, 0]), u), (u, 3 * u - 1),
+                    (np.repeat(u[:1], 40, axis=0), u)):
         bvh = bq.gpuBuilder(_cuda(boxes_np(pts)), bq.BuildConfig(makeLeafThreshold=4))
-        for k in (1, 8, 20):
-            a = bq.points.findKNN(bvh, _cuda(pts), _cuda(qs), k)
-            b = bq.points.findKNN(bvh, _cuda(pts), _cuda(qs), k, qcfg=bq.query_config(reorder=0))
-            assert _same(a, b), f"k {k}"
+        for k in (5, 16, 20):
+            _knn_both_ways(bq, bvh, _cuda(pts), _cuda(qs), k, True)
+        bvh.free()
 
 
 def test_knn_shared_search_leaves_out_unusable_queries(bq):
     """NaN, infinite and overflowing queries share a warp with ordinary ones."""
     pts = W.uniform_points(5000)
-    qs = W.uniform_points(500, 4)
+    qs = W.uniform_points(6000, 4)
     qs[::9, 0] = np.nan
     qs[4::9, 1] = np.inf
     qs[5::9, 2] = 1e30
     qs[6::9] = -np.inf
     bvh = bq.cuda.radixBuilder(_cuda(boxes_np(pts)))
-    a = bq.points.findKNN(bvh, _cuda(pts), _cuda(qs), 6)
-    b = bq.points.findKNN(bvh, _cuda(pts), _cuda(qs), 6, qcfg=bq.query_config(reorder=0))
-    assert _same(a, b)
+    for k in (6, 20):
+        ids, _, found = _knn_both_ways(bq, bvh, _cuda(pts), _cuda(qs), k, True)
+        ok = torch.from_numpy(np.abs(qs).max(1) <= 1).cuda()
+        assert bool((found[ok] == k).all()) and bool((ids[~ok] == -1).all())
 
 
 def test_batched_knn_warps_that_span_clouds(bq):
-    """Clouds with fewer than 32 queries, empty ones and one of one point."""
-    sizes, nqs = [1, 500, 0, 3, 4000, 17], [5, 40, 3, 1, 300, 31]
+    """Clouds with fewer than 32 queries, empty ones, one of one point, some
+    with enough queries a prim to share the search and some without."""
+    sizes, nqs = [1, 500, 0, 3, 400, 17, 60, 32, 2000, 33], [5, 40, 3, 1, 1000, 31, 77, 45, 1999, 700]
     pts, qs = W.uniform_points(sum(sizes)), W.uniform_points(sum(nqs), 6)
+    qs[::50] = np.nan
     off, qoff = np.concatenate([[0], np.cumsum(sizes)]), np.concatenate([[0], np.cumsum(nqs)])
     tp, tq = _cuda(pts), _cuda(qs)
     batch = bq.Batch(_cuda(boxes_np(pts)), _cuda(off))
-    for k in (1, 8, 20):
-        a = bq.batched_knn(batch, tp, _cuda(off), tq, _cuda(qoff), k)
-        b = bq.batched_knn(batch, tp, _cuda(off), tq, _cuda(qoff), k, qcfg=bq.query_config(reorder=0))
-        assert _same(a, b), f"k {k}"
+    for k in (1, 4, 5, 8, 16, 20, 32, 33):
+        for r in (float("inf"), 0.01):
+            a, ran = _phases(bq, lambda: bq.batched_knn(batch, tp, _cuda(off), tq, _cuda(qoff), k, maxSqrDist=r))
+            b = bq.batched_knn(batch, tp, _cuda(off), tq, _cuda(qoff), k, maxSqrDist=r, qcfg=bq.query_config(reorder=0))
+            assert ("batch.knn_shared" in ran) == (4 < k <= 32)
+            assert _same(a, b), f"k {k} radius {r}"
 
 
 def _mesh(level, n=None):
