@@ -15,9 +15,9 @@
 //     d sqrDist / d q   =  2 (q - X)
 //     d sqrDist / d v_k = -2 w_k (q - X).
 // Per query the three vertex contributions become (vertexID, pair index)
-// records; a stable radix sort by vertex id groups them and one thread (or, of
-// many pairs, one warp) per vertex sums its group in a fixed order.  No float atomics: the result is
-// bitwise reproducible.
+// records; a stable radix sort by vertex id groups them and one thread (four or
+// 32 of many pairs) per vertex sums its group in a fixed order.  No float
+// atomics: the result is bitwise reproducible.
 #include <algorithm>
 
 #include "bq_tri.cuh"
@@ -31,11 +31,14 @@ namespace {
 // 44.8 with 16 -- the kernel waits on its node and vertex loads, not on the
 // stack -- so none.
 constexpr int TRI_SMEM_STACK = 0;
-// Pairs a vertex (on average) from which a warp sums them, adjoint in ms by
-// thread and by warp: 18 (4M queries, 655,362 vertices) 2.29 and 1.30, 800
-// 1.64 and 0.16, 24,000 46 and 1.16; but 10 (6.4M queries, 1.9M vertices)
-// 1.50 and 3.74.
-constexpr uint32_t BWD_WARP_PAIRS = 16;
+// Pairs a vertex (on average) from which four lanes, and from which a warp,
+// sum them.  The whole adjoint, ms by one thread, four lanes and a warp a
+// vertex, pairs spread evenly and as the closest triangles of queries in a
+// cube around the mesh: 10 (2.2M queries, 655,362 vertices) 0.53 0.55 0.99 and
+// 1.16 0.62 0.98; 18 (4M) 0.88 0.86 1.29 and 2.16 1.02 1.30; 64 (14M) 3.57
+// 2.73 2.96 and 7.76 3.13 2.97; 1,852 (100,000 queries, 162 vertices) 1.64
+// 0.21 0.11 and 2.15 0.25 0.11.
+constexpr uint32_t BWD_QUAD_PAIRS = 16, BWD_WARP_PAIRS = 64;
 
 template <int TIE, typename Stack>
 __device__ __forceinline__ bool run_tri(const Node *nodes, const uint32_t *primIDs, const int32_t *tris,
@@ -200,31 +203,34 @@ __device__ __forceinline__ uint32_t first_pair(const uint32_t *__restrict__ sort
   return lo;
 }
 
-// One warp per vertex: lane l adds its pairs l, l + 32, ... in sorted order,
-// then the lanes are added pairwise; reproducible like the other, and with
-// shorter chains of additions.  For meshes with many queries a vertex, where
-// one thread's chain of dependent gathers is what takes the time.
-__global__ void k_tri_bwd_reduce_warp(const uint32_t *__restrict__ sortedKeys,
-                                      const uint32_t *__restrict__ sortedVals, uint32_t numPairs,
-                                      const float *__restrict__ contrib, uint32_t numVerts, float *__restrict__ gradV)
+// L lanes per vertex: lane l adds its pairs l, l + L, ... in sorted order, then
+// the lanes are added pairwise; reproducible like the other, and with shorter
+// chains of additions.  For meshes with many queries a vertex, where one
+// thread's chain of dependent gathers is what takes the time.
+template <int L>
+__global__ void k_tri_bwd_reduce_lanes(const uint32_t *__restrict__ sortedKeys,
+                                       const uint32_t *__restrict__ sortedVals, uint32_t numPairs,
+                                       const float *__restrict__ contrib, uint32_t numVerts, float *__restrict__ gradV)
 {
-  const uint32_t v = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (v >= numVerts) return;
+  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t lane = threadIdx.x & (L - 1);
+  const bool mine = t / L < numVerts;
+  const uint32_t v = mine ? (uint32_t)(t / L) : numVerts - 1;
   const uint32_t lo = first_pair(sortedKeys, numPairs, v), hi = first_pair(sortedKeys, numPairs, v + 1);
   float sx = 0.f, sy = 0.f, sz = 0.f;
-  for (uint32_t j = lo + lane; j < hi; j += 32) {
+  for (uint32_t j = lo + lane; j < hi; j += L) {
     const uint32_t p = sortedVals[j];
     sx += contrib[3ull * p + 0];
     sy += contrib[3ull * p + 1];
     sz += contrib[3ull * p + 2];
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = L / 2; o > 0; o >>= 1) {
     sx += __shfl_xor_sync(0xffffffffu, sx, o);
     sy += __shfl_xor_sync(0xffffffffu, sy, o);
     sz += __shfl_xor_sync(0xffffffffu, sz, o);
   }
-  if (lane == 0) {
+  if (mine && lane == 0) {
     gradV[3ull * v + 0] = sx;
     gradV[3ull * v + 1] = sy;
     gradV[3ull * v + 2] = sz;
@@ -381,7 +387,11 @@ int tri_distance_bwd(const int32_t *tris, const float *verts, uint32_t numVerts,
   int sel = 0;
   BQ_TRY(onesweep_sort_u32(keys, vals, np, nullptr, 0, bits, nullptr, &sel, err, al));
   if (numVerts && np / BWD_WARP_PAIRS >= numVerts)
-    k_tri_bwd_reduce_warp<<<div_up(numVerts, 8), 256, 0, al.s>>>(keys[sel], vals[sel], np, contrib, numVerts, gradV);
+    k_tri_bwd_reduce_lanes<32><<<div_up(32ull * numVerts, 256), 256, 0, al.s>>>(keys[sel], vals[sel], np, contrib,
+                                                                                numVerts, gradV);
+  else if (numVerts && np / BWD_QUAD_PAIRS >= numVerts)
+    k_tri_bwd_reduce_lanes<4><<<div_up(4ull * numVerts, 256), 256, 0, al.s>>>(keys[sel], vals[sel], np, contrib,
+                                                                              numVerts, gradV);
   else if (numVerts)
     k_tri_bwd_reduce<<<div_up(numVerts, 256), 256, 0, al.s>>>(keys[sel], vals[sel], np, contrib, numVerts, gradV);
   BQ_CUDA(cudaGetLastError());

@@ -312,10 +312,10 @@ def test_closest_point_where_sorting_begins(bq, tie, leaf):
         assert _same(a, [x[:nq] for x in b]), nq
 
 
-# just below and above the pairs a vertex at which a warp sums them, and many more
-@pytest.mark.parametrize("nq", [250, 863, 864, 40000])
-def test_vertex_gradients_by_thread_and_by_warp(bq, oracle, nq):
-    verts, tris = W.icosphere(2)  # 162 vertices (below 16 pairs each up to 863 queries)
+# just below and above the pairs a vertex at which four lanes sum them, and a warp, and many more
+@pytest.mark.parametrize("nq", [250, 863, 864, 3455, 3456, 40000])
+def test_vertex_gradients_by_thread_by_four_lanes_and_by_warp(bq, oracle, nq):
+    verts, tris = W.icosphere(2)  # 162 vertices (16 pairs each from 864 queries on, 64 from 3,456)
     qs = W.uniform_points(nq, 3, -1.5, 1.5)
     g = (0.5 + W.uniform_points(nq, 8)[:, 0]).astype(np.float32)
     tv, tt, tq = _cuda(verts), _cuda(tris), _cuda(qs)
