@@ -35,15 +35,21 @@ namespace {
 constexpr int SMEM_STACK = 8;
 constexpr int KNN_SMEM_STACK = 0;
 
-// Fewer queries than this are taken in the given order: the keys and the
-// sort cost 30-45 us, more than coherent warps save while the queries do not
-// fill the GPU.  Closest point, ms sorted and not: 1,001 queries 0.119 and
-// 0.083, 16,001 0.140 and 0.108, 150,001 0.177 and 0.154 (over 1M points,
-// leaves of eight: 0.225 and 0.198); 1M have to be sorted.  kNN, k = 8:
-// 1,001 0.149 and 0.124, 5,003 0.172 and 0.161, 16,001 equal, 50,001 0.205
-// and 0.313; the shared search needs the order, and with long lists it pays
-// from the start (k = 32, 1,001: 0.195 and 0.259).
-constexpr uint32_t CP_ORDER_MIN = 1u << 17;
+// Few queries are taken in the given order: the keys and the sort cost 30-45
+// us, more than coherent warps save while the queries do not fill the GPU.
+// Closest point, ms sorted and as given.  10,000 points: 160,000 queries 0.166
+// and 0.134, 250,000 0.180 and 0.156, 400,000 0.214 and 0.219; 1M points 0.193
+// 0.169, 0.220 0.207, 0.284 0.316 (leaves of eight 0.224 0.195, 0.245 0.237,
+// 0.323 0.353).  Once the nodes are far larger than L2 the order pays sooner:
+// 5M points, leaves of one (320 MB) 131,100 0.235 and 0.222, 200,000 0.255 and
+// 0.270; 7M 0.241 0.246; 10M (640 MB) 0.245 0.267, and 100,000 equal at 0.233.
+// kNN, k = 8: 1,001 0.149 and 0.124, 5,003 0.172 and 0.161, 16,001 equal,
+// 50,001 0.205 and 0.313; the shared search needs the order, and with long
+// lists it pays from the start (k = 32, 1,001: 0.195 and 0.259).
+inline bool cp_order_pays(uint32_t nq, uint32_t numNodes)
+{
+  return nq >= (1u << 18) || (nq >= (1u << 16) && (uint64_t)nq * numNodes >= 1700000000000ull);
+}
 inline uint32_t knn_order_min(int k) { return k <= 8 ? 4096 : 2; }
 // Longest lists whose searches, a thread each, do not walk in step: inserting
 // into them costs little, so leaves are better taken at once (2M points and
@@ -666,7 +672,8 @@ int closest_point(const bq_bvh3f *bvh, const float *points, const float *queries
   }
   TempSet tmp(al);
   QueryScratch qs;
-  BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0 && nq >= CP_ORDER_MIN, false, tmp, al, qs));
+  BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0 && cp_order_pays(nq, bvh->numNodes), false,
+                         tmp, al, qs));
   const int tie = c.tieMode, st = c.stackDepth, b = c.blockSize;
   if (tie == BQ_TIES_REFERENCE) {
     if (st == 32) launch_cp<TIE_REFERENCE, 32>(bvh, points, queries, nq, maxSqr, b, ids, d, qs, al.s, ex);

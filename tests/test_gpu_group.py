@@ -304,12 +304,26 @@ def test_closest_point_where_sorting_begins(bq, tie, leaf):
     that are processed at once and in step."""
     pts = W.uniform_points(30000)
     tp = _cuda(pts)
-    qs = _cuda(W.uniform_points(131073, W.SEED_QUERIES, -0.1, 1.1))
+    qs = _cuda(W.uniform_points(262145, W.SEED_QUERIES, -0.1, 1.1))
     bvh = bq.gpuBuilder(_cuda(boxes_np(pts)), bq.BuildConfig(makeLeafThreshold=leaf))
     b = bq.points.findClosest(bvh, tp, qs, qcfg=bq.query_config(tieMode=tie, reorder=0))
-    for nq in (1, 33, 131071, 131072, 131073):
-        a = bq.points.findClosest(bvh, tp, qs[:nq], qcfg=bq.query_config(tieMode=tie))
-        assert _same(a, [x[:nq] for x in b]), nq
+    for nq in (1, 33, 262143, 262144, 262145):
+        a, ran = _phases(bq, lambda: bq.points.findClosest(bvh, tp, qs[:nq], qcfg=bq.query_config(tieMode=tie)))
+        assert _same(a, [x[:nq] for x in b]) and ("query.keys" in ran) == (nq >= 262144), nq
+
+
+def test_closest_point_over_many_nodes_is_sorted_sooner(bq):
+    g = torch.Generator(device="cuda").manual_seed(2)
+    tp = torch.rand((4_000_000, 3), generator=g, device="cuda")
+    bvh = bq.cuda.radixBuilder(bq.points_to_boxes(tp))
+    first = -(-1_700_000_000_000 // bvh.numNodes)
+    assert 1 << 16 < first < 1 << 18
+    qs = torch.rand((first, 3), generator=g, device="cuda")
+    b = bq.points.findClosest(bvh, tp, qs, qcfg=bq.query_config(reorder=0))
+    for nq in (first - 1, first):
+        a, ran = _phases(bq, lambda: bq.points.findClosest(bvh, tp, qs[:nq]))
+        assert _same(a, [x[:nq] for x in b]) and ("query.keys" in ran) == (nq == first), nq
+    bvh.free()
 
 
 # just below and above the pairs a vertex at which four lanes sum them, and a warp, and many more
