@@ -105,6 +105,48 @@ __device__ __forceinline__ bool box_traverse(const Node *__restrict__ nodes, con
   }
 }
 
+// The same by each lane on its own.
+template <typename Fn>
+__device__ __forceinline__ bool box_traverse_alone(const Node *__restrict__ nodes, const uint32_t *__restrict__ primIDs,
+                                                   const bq_box3f *__restrict__ boxes, const float q[6], Fn &fn)
+{
+  uint64_t stack[BOX_STACK];
+  int sp = 0;
+  uint64_t admin = node_admin(ldg_node(nodes));
+  while (true) {
+    bool leaf = true;
+    while (admin_count(admin) == 0) {
+      const uint64_t off = admin_offset(admin);
+      const Node n0 = ldg_node(nodes + off), n1 = ldg_node(nodes + off + 1);
+      const bool o0 = box_overlaps(q, n0.a.x, n0.a.y, n0.a.z, n0.a.w, n0.b.x, n0.b.y);
+      const bool o1 = box_overlaps(q, n1.a.x, n1.a.y, n1.a.z, n1.a.w, n1.b.x, n1.b.y);
+      if (o0) {
+        if (o1) {
+          if (sp >= BOX_STACK) return false;
+          stack[sp++] = node_admin(n1);
+        }
+        admin = node_admin(n0);
+      } else if (o1) {
+        admin = node_admin(n1);
+      } else {
+        leaf = false;
+        break;
+      }
+    }
+    if (leaf) {
+      const uint64_t off = admin_offset(admin);
+      const uint32_t cnt = admin_count(admin);
+      for (uint32_t j = 0; j < cnt; j++) {
+        const uint32_t pid = __ldg(primIDs + off + j);
+        const bq_box3f b = boxes[pid];
+        if (box_overlaps(q, b.lower[0], b.lower[1], b.lower[2], b.upper[0], b.upper[1], b.upper[2])) fn(pid);
+      }
+    }
+    if (sp == 0) return true;
+    admin = stack[--sp];
+  }
+}
+
 // fixedBoxQuery::forEachLeaf over a WideBVH (:161-230), same contract as
 // box_traverse.  A stack entry is (wide node << 8 | slot to resume at).
 template <int W, typename Fn>
@@ -148,14 +190,19 @@ __device__ __forceinline__ bool wide_box_traverse(const Node *__restrict__ slots
   }
 }
 
-// W == 0: binary tree (the warp together), else a W-wide tree (each lane
-// with a query by itself)
+// W == 0: binary tree (the warp together), BOX_ALONE: binary tree (each lane
+// with a query by itself), else a W-wide tree (likewise).  With one to three
+// queries there is nobody to wait for: one box with most of 2M points, count
+// and ids 1,189 ms together, 997 alone; two 726 and 696, eight 489 and 744.
+constexpr int BOX_ALONE = -1;
+constexpr uint32_t BOX_STEP_MIN = 4;
 template <int W, typename Fn>
 __device__ __forceinline__ bool any_box_traverse(const Node *__restrict__ nodes, const uint32_t *__restrict__ primIDs,
                                                  const bq_box3f *__restrict__ boxes, const float q[6], Fn &fn,
                                                  bool alive)
 {
   if constexpr (W == 0) return box_traverse(nodes, primIDs, boxes, q, fn, alive);
+  else if constexpr (W == BOX_ALONE) return !alive || box_traverse_alone(nodes, primIDs, boxes, q, fn);
   else return !alive || wide_box_traverse<W>(nodes, primIDs, boxes, q, fn);
 }
 
@@ -366,10 +413,10 @@ int box_query_order(const Node *nodes, const bq_box3f *queryBoxes, uint32_t nq, 
   *order = nullptr;
   if (nq < BOX_ORDER_MIN) return BQ_OK;
   const float *rootBox = (const float *)nodes;  // binary: the root node's box
-  if (W != 0) {
+  if (W > 0) {
     float *rb = nullptr;
     BQ_TRY(tmp.get(&rb, 6));
-    launch_pdl(k_wide_root_box<W == 0 ? 2 : W>, dim3(1), dim3(32), 0, al.s, nodes, rb);
+    launch_pdl(k_wide_root_box<(W > 0 ? W : 2)>, dim3(1), dim3(32), 0, al.s, nodes, rb);
     rootBox = rb;
   }
   uint32_t *keys[2], *idx[2];
@@ -454,7 +501,10 @@ int box_query_slab(const bq_bvh3f *bvh, const bq_box3f *boxes, const bq_box3f *q
     BQ_CUDA(cudaMemsetAsync(ovf, 0, 4, al.s));
     return BQ_OK;
   }
-  return slab_impl<0>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, slabCap, slab, counts, ovf, al);
+  return nq < BOX_STEP_MIN ? slab_impl<BOX_ALONE>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, slabCap,
+                                                  slab, counts, ovf, al)
+                           : slab_impl<0>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, slabCap, slab,
+                                          counts, ovf, al);
 }
 
 int box_query_gather(const bq_bvh3f *bvh, const bq_box3f *boxes, const bq_box3f *queryBoxes, uint32_t nq,
@@ -462,8 +512,10 @@ int box_query_gather(const bq_bvh3f *bvh, const bq_box3f *boxes, const bq_box3f 
                      const uint32_t *offsets, uint64_t capacity, int32_t *ids, Alloc &al)
 {
   if (nq == 0 || bvh->numNodes == 0) return BQ_OK;
-  return gather_impl<0>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, slabCap, slab, counts, ovf,
-                        offsets, capacity, ids, al);
+  return nq < BOX_STEP_MIN ? gather_impl<BOX_ALONE>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq,
+                                                    slabCap, slab, counts, ovf, offsets, capacity, ids, al)
+                           : gather_impl<0>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, slabCap,
+                                            slab, counts, ovf, offsets, capacity, ids, al);
 }
 
 int wide_box_query_slab(const bq_wide_bvh3f *bvh, int W, const bq_box3f *boxes, const bq_box3f *queryBoxes,
@@ -504,14 +556,19 @@ int box_query_count(const bq_bvh3f *bvh, const bq_box3f *boxes, const bq_box3f *
     BQ_CUDA(cudaMemsetAsync(counts, 0, sizeof(uint32_t) * nq, al.s));
     return BQ_OK;
   }
-  return count_impl<0>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, counts, al);
+  return nq < BOX_STEP_MIN
+             ? count_impl<BOX_ALONE>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, counts, al)
+             : count_impl<0>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, counts, al);
 }
 
 int box_query_fill(const bq_bvh3f *bvh, const bq_box3f *boxes, const bq_box3f *queryBoxes, uint32_t nq,
                    const uint32_t *offsets, uint64_t capacity, int32_t *ids, Alloc &al)
 {
   if (nq == 0 || bvh->numNodes == 0) return BQ_OK;
-  return fill_impl<0>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, offsets, capacity, ids, al);
+  return nq < BOX_STEP_MIN
+             ? fill_impl<BOX_ALONE>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, offsets, capacity,
+                                    ids, al)
+             : fill_impl<0>((const Node *)bvh->nodes, bvh->primIDs, boxes, queryBoxes, nq, offsets, capacity, ids, al);
 }
 
 int wide_box_query_count(const bq_wide_bvh3f *bvh, int W, const bq_box3f *boxes, const bq_box3f *queryBoxes,

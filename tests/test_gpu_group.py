@@ -278,9 +278,9 @@ def test_triangle_groups_heavy_queries(bq):
     assert np.allclose(((p[ok] - qs[ok]) ** 2).sum(1), d[ok], rtol=1e-5)
 
 
-# one warp, parts of one, more than one; above 16,384 queries are sorted.  A row of 3 ids sends most queries to the
-# second traversal.
-@pytest.mark.parametrize("nq", [1, 31, 33, 129, 16385])
+# below four queries each lane is on its own; one warp, parts of one, more than one; above 16,384 queries are sorted.
+# A row of 3 ids sends most queries to the second traversal.
+@pytest.mark.parametrize("nq", [1, 3, 4, 31, 33, 129, 16385])
 @pytest.mark.parametrize("leaf", [1, 8])
 def test_box_queries_of_partial_warps_match_oracle(bq, oracle, nq, leaf):
     pts = W.uniform_points(6000)
