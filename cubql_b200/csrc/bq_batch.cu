@@ -538,14 +538,18 @@ __global__ void k_seg_knn_deep(const bq_bvh3f *__restrict__ bvhs, const uint32_t
 constexpr int DEEP_THREADS = 2048;
 constexpr int DEEP_STACK = 1024;
 
+// lists whose clouds may be searched a warp at a time (short ones are found
+// sooner by a thread, as densities are known cloud by cloud only)
+constexpr bool seg_shared(int k) { return k > 4 && k <= 32; }
+
 template <int K, int TIE, int STACK>
 int launch_seg_knn(const bq_bvh3f *bvhs, const uint32_t *poff, const float *points, const float *queries,
                    const uint32_t *qoff, const uint64_t *skeys, const uint32_t *order, uint32_t nq, int k, float maxSqr,
                    int block, int chunk, uint32_t *workCtr, int32_t *ids, float *d, int32_t *nf, uint32_t *ovfList,
                    uint32_t *ovfCount, StackEntry *deep, uint32_t *leftList, uint32_t *err, cudaStream_t s)
 {
-  if (TIE == TIE_LOWEST && K > 4 && K <= 32 && order) {
-    constexpr int KK = K > 4 && K <= 32 ? K : 32;
+  if (TIE == TIE_LOWEST && seg_shared(K) && order) {
+    constexpr int KK = seg_shared(K) ? K : 32;
     {
       ProfScope ps("batch.knn_shared", s);
       launch_pdl(k_seg_knn_warp<KK>, dim3(div_up(nq, block)), dim3(block), 0, s, bvhs, poff, points, queries, qoff,
@@ -776,6 +780,7 @@ int autotune_batched_knn(const bq_box3f *boxes, const float *points, const uint3
     for (int st : stacks)
       for (int bl : blocks)
         for (int gr : grabs) {
+          if (gr != 32 && seg_shared(k)) continue;  // the shared search takes no grabs
           bq_query_config qc{BQ_TIES_LOWEST_ID, st, bl, 1, gr};
           float tb = 0.f, tq = 0.f;
           for (int rep = 0; rep < 2 && status == BQ_OK; rep++) {  // rep 0 warms up

@@ -688,6 +688,13 @@ int closest_point(const bq_bvh3f *bvh, const float *points, const float *queries
   return finish_queries(qs, al);
 }
 
+// whether one search serves a warp's 32 queries (launch_knn)
+bool knn_is_shared(uint32_t nq, uint32_t numPrims, int k, const bq_query_config &c)
+{
+  return c.tieMode == BQ_TIES_LOWEST_ID && k >= 1 && k <= 32 && c.lanesPerQuery <= 1 && c.reorder &&
+         nq >= knn_order_min(k) && group_pays(nq, numPrims, k);
+}
+
 int knn(const bq_bvh3f *bvh, const float *points, const float *queries, uint32_t nq, int k, float maxSqr,
         const bq_query_config *qcfg, int32_t *ids, float *d, int32_t *numFound, Alloc &al)
 {
@@ -702,11 +709,9 @@ int knn(const bq_bvh3f *bvh, const float *points, const float *queries, uint32_t
   }
   TempSet tmp(al);
   QueryScratch qs;
-  // one search for a warp's queries (launch_knn); its order is the curve
-  // without jumps
-  const bool shared =
-      c.tieMode == BQ_TIES_LOWEST_ID && k <= 32 && c.lanesPerQuery == 1 && group_pays(nq, bvh->numPrims, k);
-  BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0 && nq >= knn_order_min(k), shared, tmp, al, qs));
+  const bool shared = knn_is_shared(nq, bvh->numPrims, k, c);  // its order is the curve without jumps
+  BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0 && nq >= knn_order_min(k), shared, tmp,
+                         al, qs));
   const int tie = c.tieMode, st = c.stackDepth, b = c.blockSize;
   if (c.lanesPerQuery > 1) {
     if (k > c.lanesPerQuery) return set_error(BQ_ERR_INVALID_ARGUMENT, "lanesPerQuery must be at least k");

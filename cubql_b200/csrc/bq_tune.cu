@@ -5,7 +5,9 @@
 // size is timed with CUDA events on the caller's inputs (a Morton build of
 // the boxes, then one query batch; one warm-up each), and the fastest
 // build + query is returned.  With the default tie rule the answers do not
-// depend on these knobs, only the time.
+// depend on these knobs, only the time.  Where the shared kNN search runs,
+// which has a stack of its own, the depth is not varied: it would only reach
+// the few queries that the search leaves, and the choice be noise.
 #include <cmath>
 
 #include "bq_internal.cuh"
@@ -17,6 +19,8 @@ int closest_point(const bq_bvh3f *bvh, const float *points, const float *queries
                   int excludeSelf);
 int knn(const bq_bvh3f *bvh, const float *points, const float *queries, uint32_t nq, int k, float maxSqr,
         const bq_query_config *qcfg, int32_t *ids, float *d, int32_t *numFound, Alloc &al);
+
+bool knn_is_shared(uint32_t nq, uint32_t numPrims, int k, const bq_query_config &c);
 
 namespace {
 // mean ms of `reps` runs of fn after one warm-up, CUDA events on the stream
@@ -82,6 +86,7 @@ int autotune_query(const bq_box3f *boxes, const float *points, uint32_t n, const
       for (int bl : blocks) {
         if (status != BQ_OK) break;
         const bq_query_config qc{BQ_TIES_LOWEST_ID, st, bl, 1, 32};
+        if (st != 64 && knn_is_shared(nq, t.numPrims, k, qc)) continue;
         float tq = 0.f;
         status = time_ms(
             [&]() -> int {

@@ -482,8 +482,9 @@ int bq_batched_tri_closest_f3(const bq_bvh3f *bvhs, const uint32_t *triOffsets, 
 
 /* Launch-shape autotuner for a batched build + kNN workload: times every
    combination of leaf threshold {1,2,4,8}, stack depth {32,64}, block
-   size {64,128} and queries per warp {32,128} on the given inputs (CUDA
-   events, after one warm-up) and returns the fastest.  With the default
+   size {64,128} and queries per warp ({32,128}; 32 alone for k of 5 to 32,
+   where it has no effect) on the given inputs (CUDA events, after one
+   warm-up) and returns the fastest.  With the default
    tie rule the answers do not depend on these knobs, only the time. */
 typedef struct bq_tuning {
   int makeLeafThreshold;
@@ -500,9 +501,9 @@ int bq_autotune_batched_knn_f3(const bq_box3f *boxes, const float *points, const
 
 /* The same for one tree: Morton builds with leaf threshold {1,2,4,8},
    each queried with stack depth {32,64,128} x block size {64,128}, closest
-   point (k == 0) or kNN (k in [1, 64]); best->queriesPerWarp is 32 (the
-   single-tree kernels take one query per thread).  The fastest build +
-   query is returned with its two times. */
+   point (k == 0) or kNN (k in [1, 64]); stack depth stays 64 where one search
+   serves a warp's queries, and best->queriesPerWarp is 32.  The fastest build
+   + query is returned with its two times. */
 int bq_autotune_query_f3(const bq_box3f *boxes, const float *points, uint32_t numPrims, const float *queries,
                          uint32_t numQueries, int k, bq_tuning *best, const bq_allocator *alloc, bq_stream_t stream);
 

@@ -35,3 +35,22 @@ def test_tuned_query_shape_and_answers(bq, tmp_path, k):
         a = bq.points.findKNN(bvh, tp, qs, k, qcfg=qc)[:2]
         r = bq.points.findKNN(ref, tp, qs, k)[:2]
     assert all(torch.equal(x, y) for x, y in zip(a, r))
+
+
+@pytest.mark.parametrize("nq,shapes", [(100_000, 4 * 2), (1000, 4 * 6)])
+def test_only_knobs_that_act_are_tuned(bq, nq, shapes):
+    """Where the shared kNN search runs, stack depth (one tree) and queries
+    a grab (a batch) reach none of its launches and are not varied."""
+    import ctypes
+    pts, qs = W.uniform_points(20_000), W.uniform_points(nq, W.SEED_QUERIES)
+    b, tp, tq = (torch.from_numpy(x).cuda() for x in (boxes_np(pts), pts, qs))
+    best = bq.bq_tuning()
+    with bq.profile() as prof:
+        bq._check(bq._lib.bq_autotune_query_f3(bq._ptr(b), bq._ptr(tp), len(pts), bq._ptr(tq), nq, 16,
+                                               ctypes.byref(best), None, bq._stream()))
+    assert prof.table["query.knn_shared" if nq == 100_000 else "query.knn"][0] == shapes * 3  # a warm-up, two timed
+    off = torch.tensor([0, 5000, 20_000], dtype=torch.int32)
+    for k, phase, grabs in ((16, "batch.knn_shared", 1), (4, "batch.knn", 2)):
+        with bq.profile() as prof:
+            t = bq.autotune_batched_knn(b, tp, off, tq, torch.tensor([0, nq // 2, nq], dtype=torch.int32), k)
+        assert prof.table[phase][0] == 4 * 2 * 2 * grabs * 2 and t["queriesPerWarp"] in (32, 128)[:grabs]
