@@ -45,17 +45,6 @@ int query_config(const bq_query_config *q, bq_query_config &out);
 
 namespace {
 
-__device__ __forceinline__ uint32_t seg_of(const uint32_t *__restrict__ off, uint32_t numSegs, uint32_t i)
-{
-  // largest s with off[s] <= i
-  uint32_t lo = 0, hi = numSegs;
-  while (hi - lo > 1) {
-    const uint32_t m = (lo + hi) >> 1;
-    if (__ldg(off + m) <= i) lo = m; else hi = m;
-  }
-  return lo;
-}
-
 // box center (lower + upper) / 2, as a multiply by 0.5: the same float
 __device__ __forceinline__ float ctr(float lo, float hi) { return __fmul_rn(__fadd_rn(lo, hi), 0.5f); }
 
@@ -337,25 +326,6 @@ struct BKnnLeaf {
   }
 };
 
-template <int K, int TIE>
-__device__ __forceinline__ void write_knn(const KnnList<K, TIE> &list, uint32_t qi, int k, int32_t *outIds,
-                                          float *outD, int32_t *numFound)
-{
-  int found = 0;
-  int32_t *oi = outIds + (size_t)qi * k;
-  float *od = outD + (size_t)qi * k;
-#pragma unroll
-  for (int j = 0; j < K; j++) {
-    if (j >= K - k) {
-      const bool real = list.real(j);
-      oi[j - (K - k)] = real ? list.id(j) : -1;
-      od[j - (K - k)] = real ? list.dist(j) : INFINITY;
-      found += real ? 1 : 0;
-    }
-  }
-  if (numFound) numFound[qi] = found;
-}
-
 // one search for a warp's 32 queries (bq_group.cuh), or one for each cloud
 // that they belong to; queries that cannot share it go on a list (of places
 // in the visiting order), with what is known of their k-th best distance in
@@ -535,8 +505,6 @@ __global__ void k_seg_knn_deep(const bq_bvh3f *__restrict__ bvhs, const uint32_t
   }
 }
 
-constexpr int DEEP_THREADS = 2048;
-constexpr int DEEP_STACK = 1024;
 
 // lists whose clouds may be searched a warp at a time (short ones are found
 // sooner by a thread, as densities are known cloud by cloud only)

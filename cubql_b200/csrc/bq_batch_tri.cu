@@ -27,7 +27,7 @@ constexpr uint32_t BR_NO_PARENT = 0xffffffffu;
 __device__ __forceinline__ bool node_slot(const bq_bvh3f *__restrict__ bvhs, const uint32_t *__restrict__ off,
                                           uint32_t numSegs, uint32_t j, uint32_t &s, uint32_t &local)
 {
-  s = seg_find(off, numSegs, j >> 1);
+  s = seg_of(off, numSegs, j >> 1);
   local = j - 2 * __ldg(off + s);
   return local < bvhs[s].numNodes;
 }
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(128) k_btri(const bq_bvh3f *__restrict__ bvhs,
   griddep_wait();
   const uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x;
   if (qi >= nq) return;
-  const uint32_t s = seg_find(qoff, numSegs, qi);
+  const uint32_t s = seg_of(qoff, numSegs, qi);
   const bq_bvh3f d = bvhs[s];
   LocalStack<STACK> st;
   if (!run_btri<TIE>(d, __ldg(triOff + s), tris, verts, queries, qi, maxSqr, st, outIds, outD, outP))
@@ -149,7 +149,7 @@ __global__ void k_btri_deep(const bq_bvh3f *__restrict__ bvhs, const uint32_t *_
   const uint32_t cnt = *ovfCount;
   for (uint32_t w = tid; w < cnt; w += gridDim.x * blockDim.x) {
     const uint32_t qi = ovfList[w];
-    const uint32_t s = seg_find(qoff, numSegs, qi);
+    const uint32_t s = seg_of(qoff, numSegs, qi);
     GlobalStack st{stacks + (size_t)tid * DEEP_STACK, DEEP_STACK, 0};
     if (!run_btri<TIE>(bvhs[s], triOff[s], tris, verts, queries, qi, maxSqr, st, outIds, outD, outP)) {
       outIds[qi] = -1;
@@ -168,7 +168,7 @@ __global__ void k_btri_keys(const bq_bvh3f *__restrict__ bvhs, const float *__re
   griddep_wait();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nq) return;
-  const uint32_t s = seg_find(qoff, numSegs, t);
+  const uint32_t s = seg_of(qoff, numSegs, t);
   const bq_bvh3f d = bvhs[s];
   const uint32_t h = d.numNodes ? query_order_key((const float *)d.nodes, queries + 3ull * t) : 0;
   keys[t] = (uint32_t)((((uint64_t)s << 30) | h) >> max(segBits - 2, 0));

@@ -404,7 +404,7 @@ int fill_impl(const Node *nodes, const uint32_t *primIDs, const bq_box3f *boxes,
   return BQ_OK;
 }
 
-// visiting order of nq query boxes along a Morton curve of their centres
+// visiting order of nq query boxes along a Hilbert curve of their centres
 // (nullptr: the given order, for few queries)
 template <int W>
 int box_query_order(const Node *nodes, const bq_box3f *queryBoxes, uint32_t nq, uint32_t *err, TempSet &tmp,

@@ -268,6 +268,17 @@ __host__ __device__ __forceinline__ uint32_t spread10(uint32_t x)
   return x;
 }
 
+// the segment of entry i: the largest s with off[s] <= i
+__device__ __forceinline__ uint32_t seg_of(const uint32_t *__restrict__ off, uint32_t numSegs, uint32_t i)
+{
+  uint32_t lo = 0, hi = numSegs;
+  while (hi - lo > 1) {
+    const uint32_t m = (lo + hi) >> 1;
+    if (__ldg(off + m) <= i) lo = m; else hi = m;
+  }
+  return lo;
+}
+
 // Position of a cell of the 1024^3 grid along a 3D Hilbert curve (30 bits;
 // Skilling, "Programming the Hilbert curve", 2004: undo the excess work of
 // each level, then Gray-encode).  Consecutive cells of this curve are

@@ -5,7 +5,8 @@
 // cuBQL/queries/points/knn.h:75-116 findKNN) that user kernels call one
 // thread per query in input order.  Here one call answers a whole batch:
 //
-//   k_query_keys   30-bit Hilbert position of every query in the root box
+//   k_query_keys   30-bit position of every query in the root box, along a
+//                  Hilbert curve for k_knn_warp, a Morton curve otherwise
 //   onesweep sort  queries reordered along the curve (top 24 key bits),
 //                  so neighbouring threads walk nearly the same nodes
 //                  (L1/L2 reuse, less divergence)
@@ -152,25 +153,6 @@ struct KnnLeaf {
     return fminf(maxSqr, list.worst());
   }
 };
-
-template <int K, int TIE>
-__device__ __forceinline__ void write_knn(const KnnList<K, TIE> &list, uint32_t qi, int k, int32_t *outIds,
-                                          float *outD, int32_t *numFound)
-{
-  int found = 0;
-  int32_t *oi = outIds + (size_t)qi * k;
-  float *od = outD + (size_t)qi * k;
-#pragma unroll
-  for (int j = 0; j < K; j++) {
-    if (j >= K - k) {
-      const bool real = list.real(j);
-      oi[j - (K - k)] = real ? list.id(j) : -1;
-      od[j - (K - k)] = real ? list.dist(j) : INFINITY;
-      found += real ? 1 : 0;
-    }
-  }
-  if (numFound) numFound[qi] = found;
-}
 
 // seed: an upper bound of the k-th best squared distance (maxSqr: none)
 // WARP: the whole warp calls together (lanes without a query: alive ==
@@ -593,6 +575,13 @@ __global__ void k_fill_empty(uint32_t nq, int k, int32_t *ids, float *d, int32_t
   if (numFound && t < nq) numFound[t] = 0;
 }
 
+void query_keys(const float *rootBox, const float *queries, uint32_t nq, bool hilbert, uint32_t *keys, uint32_t *idx,
+                cudaStream_t s)
+{
+  launch_pdl(hilbert ? k_query_keys<true> : k_query_keys<false>, dim3(div_up(nq, 256)), dim3(256), 0, s, rootBox, queries,
+             nq, keys, idx);
+}
+
 int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, bool reorder, bool hilbert, TempSet &tmp,
                     Alloc &al, QueryScratch &qs)
 {
@@ -609,8 +598,7 @@ int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, boo
     BQ_TRY(tmp.get(&idx[1], nq));
     {
       ProfScope ps("query.keys", al.s);
-      launch_pdl(hilbert ? k_query_keys<true> : k_query_keys<false>, dim3(div_up(nq, 256)), dim3(256), 0, al.s, rootBox,
-                 queries, nq, keys[0], idx[0]);
+      query_keys(rootBox, queries, nq, hilbert, keys[0], idx[0], al.s);
     }
     BQ_CUDA(cudaGetLastError());
     int sel = 0;

@@ -7,9 +7,6 @@
 
 namespace bq {
 
-constexpr int DEEP_THREADS = 2048;  // threads of a deep-stack re-run kernel
-constexpr int DEEP_STACK = 1024;    // entries of 8 bytes per deep stack
-
 // ------------------------------------------------------------------
 // closest point candidates
 // ------------------------------------------------------------------
@@ -52,13 +49,17 @@ struct CpExclude {
 struct QueryScratch {
   uint32_t *order = nullptr;
   uint32_t *ovfList = nullptr, *ovfCount = nullptr, *err = nullptr;
-  uint32_t *leftList = nullptr;  // nq words (with `order` only)
+  uint32_t *leftList = nullptr;  // nq words (with a Hilbert order only)
   StackEntry *deep = nullptr;
 };
 
+// Keys and indices of the queries for a sort along a 30-bit curve inside
+// rootBox (6 device floats: lower xyz, upper xyz): Hilbert where lanes share a
+// search, as its runs fill compact boxes, else Morton.
+void query_keys(const float *rootBox, const float *queries, uint32_t nq, bool hilbert, uint32_t *keys, uint32_t *idx,
+                cudaStream_t s);
 // Allocates the call's scratch from `tmp` and, with `reorder`, sorts the
-// queries along a 30-bit Morton curve inside rootBox (6 device floats:
-// lower xyz, upper xyz); qs.order is then the visiting order.
+// queries along that curve; qs.order is then the visiting order.
 int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, bool reorder, bool hilbert, TempSet &tmp,
                     Alloc &al, QueryScratch &qs);
 // Synchronises the stream and turns the device error word into a status.

@@ -25,6 +25,9 @@ struct StackEntry {
   float dist;
 };
 
+constexpr int DEEP_THREADS = 2048;  // threads of a deep-stack re-run kernel
+constexpr int DEEP_STACK = 1024;    // entries of 8 bytes per deep stack
+
 // fixed-size stack in local memory
 template <int N>
 struct LocalStack {
@@ -378,5 +381,25 @@ struct KnnList<K, TIE_LOWEST> {
     }
   }
 };
+
+// the k results of query qi, and how many of them there are
+template <int K, int TIE>
+__device__ __forceinline__ void write_knn(const KnnList<K, TIE> &list, uint32_t qi, int k, int32_t *outIds,
+                                          float *outD, int32_t *numFound)
+{
+  int found = 0;
+  int32_t *oi = outIds + (size_t)qi * k;
+  float *od = outD + (size_t)qi * k;
+#pragma unroll
+  for (int j = 0; j < K; j++) {
+    if (j >= K - k) {
+      const bool real = list.real(j);
+      oi[j - (K - k)] = real ? list.id(j) : -1;
+      od[j - (K - k)] = real ? list.dist(j) : INFINITY;
+      found += real ? 1 : 0;
+    }
+  }
+  if (numFound) numFound[qi] = found;
+}
 
 } // namespace bq

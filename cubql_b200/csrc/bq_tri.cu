@@ -20,6 +20,7 @@
 // atomics: the result is bitwise reproducible.
 #include <algorithm>
 
+#include "bq_query.cuh"
 #include "bq_tri.cuh"
 
 namespace bq {
@@ -116,15 +117,6 @@ __global__ void __launch_bounds__(128) k_tri_visit_count(const Node *__restrict_
     prims = cl.prims;
   }
   add_visit_counts(vc.pairs, vc.admins, prims, out);
-}
-
-__global__ void k_tri_keys(const Node *__restrict__ nodes, const float *__restrict__ queries, uint32_t nq,
-                           uint32_t *__restrict__ keys, uint32_t *__restrict__ idx)
-{
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nq) return;
-  keys[t] = query_order_key((const float *)nodes, queries + 3ull * t);
-  idx[t] = t;
 }
 
 __global__ void k_tri_fill_empty(uint32_t nq, int32_t *ids, float *d, float *P)
@@ -304,7 +296,11 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
     BQ_TRY(tmp.get(&keys[1], nq));
     BQ_TRY(tmp.get(&idx[0], nq));
     BQ_TRY(tmp.get(&idx[1], nq));
-    k_tri_keys<<<div_up(nq, 256), 256, 0, al.s>>>(nodes, queries, nq, keys[0], idx[0]);
+    {
+      ProfScope ps("tri.keys", al.s);
+      query_keys((const float *)nodes, queries, nq, true, keys[0], idx[0], al.s);
+    }
+    BQ_CUDA(cudaGetLastError());
     int sel = 0;
     BQ_TRY(onesweep_sort_u32(keys, idx, nq, nullptr, 6, 30, nullptr, &sel, err, al));  // order only: top 24 bits
     order = idx[sel];

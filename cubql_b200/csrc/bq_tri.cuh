@@ -39,9 +39,6 @@
 
 namespace bq {
 
-constexpr int DEEP_THREADS = 2048;  // threads of a deep-stack re-run kernel
-constexpr int DEEP_STACK = 1024;    // entries of 8 bytes per deep stack
-
 // fewer queries are taken in the given order: sorting costs more than it
 // saves (20,480 triangles, forward and adjoint, ms sorted and not: 5,003
 // queries 0.579 and 0.500, 16,001 0.607 and 0.526, 50,001 0.736 and 0.701,
@@ -247,16 +244,6 @@ struct TriMesh {
   const float *verts;
 };
 
-__device__ __forceinline__ uint32_t seg_find(const uint32_t *__restrict__ off, uint32_t numSegs, uint32_t i)
-{
-  uint32_t lo = 0, hi = numSegs;
-  while (hi - lo > 1) {
-    const uint32_t m = (lo + hi) >> 1;
-    if (__ldg(off + m) <= i) lo = m; else hi = m;
-  }
-  return lo;
-}
-
 // the triangle at leaf position `slot` of a tree whose first triangle is
 // `base`; key: where it competes
 __device__ __forceinline__ TriHit tri_test(const TriMesh &m, const uint32_t *primIDs, uint32_t base, uint32_t slot,
@@ -358,7 +345,7 @@ __device__ __forceinline__ void tri_group(const TriMesh &m, const float *__restr
       qmax = abs_max(q);
       bool seeded = id >= 0;
       if (m.bvhs) {
-        const uint32_t s = seg_find(m.queryOff, m.numSegs, qi);
+        const uint32_t s = seg_of(m.queryOff, m.numSegs, qi);
         seeded = seeded && s == seg;
         seg = s;
         const bq_bvh3f d = m.bvhs[s];
@@ -564,7 +551,7 @@ __global__ void __launch_bounds__(128) k_tri_near(TriMesh m, const float *__rest
   uint32_t base = 0;
   bool tree = true;
   if (m.bvhs) {
-    const uint32_t s = seg_find(m.queryOff, m.numSegs, qi);
+    const uint32_t s = seg_of(m.queryOff, m.numSegs, qi);
     const bq_bvh3f d = m.bvhs[s];
     if (__all_sync(0xffffffffu, d.numPrims > TRI_NEAR_PRIMS) && rounds != TRI_ALL) rounds = 0;
     nodes = (const Node *)d.nodes;
