@@ -127,7 +127,7 @@ def test_triangle_groups_do_not_depend_on_batch_or_tree(bq, n, nq):
     leaf order or fetched through the index), on a tree of another shape and
     in a batch; and no farther than under the reference's rule."""
     tv, tt = _mesh(5, n)
-    qs = _cuda(W.uniform_points(20000, W.SEED_QUERIES, -1.5, 1.5))
+    qs = _cuda(W.uniform_points(40000, W.SEED_QUERIES, -1.5, 1.5))  # enough to be sorted, too few for threads first
     boxes = bq.triangles.boxes(tt, tv)
     bvh, sah = bq.cuda.radixBuilder(boxes), bq.cuda.sahBuilder(boxes, bq.BuildConfig(makeLeafThreshold=3))
     for r in (float("inf"), 0.05):
@@ -137,7 +137,7 @@ def test_triangle_groups_do_not_depend_on_batch_or_tree(bq, n, nq):
         assert _same(bq.triangles.findClosest(sah, tt, tv, qs[:nq], maxSqrDist=r)[:2], few[:2])
         ref = bq.triangles.findClosest(bvh, tt, tv, qs, maxSqrDist=r, qcfg=bq.query_config(tieMode=1))
         assert bool((many[1] <= ref[1]).all()) and float((many[1] == ref[1]).float().mean()) > 0.99
-        off, qoff = _cuda(np.array([0, n, n])), _cuda(np.array([0, 20000, 20000]))
+        off, qoff = _cuda(np.array([0, n, n])), _cuda(np.array([0, 40000, 40000]))
         batch = bq.Batch(boxes, off)
         for reorder in (0, 1):
             got = bq.batched_tri_closest(batch, tt, tv, qs, qoff, maxSqrDist=r, qcfg=bq.query_config(reorder=reorder))
@@ -216,6 +216,47 @@ def test_triangle_threads_before_groups(bq, n, nq):
         many = bq.triangles.findClosest(bvh, tt, tv, tq, maxSqrDist=r)
         few = [torch.cat(x) for x in zip(*[bq.triangles.findClosest(bvh, tt, tv, q, maxSqrDist=r) for q in tq.split(30_000)])]
         assert _same(few, many), f"radius {r}"
+
+
+@pytest.mark.parametrize("nq", [300_000, 1_100_000])
+def test_batched_triangles_sorted_and_seeded(bq, oracle, nq):
+    """Meshes too large for a thread a query (its groups start from their
+    neighbour's triangle, and drop it where the mesh changes), small ones and
+    empty ones, in one sorted batch: as their queries in small calls, and as
+    an FP64 brute force."""
+    rng = np.random.default_rng(nq)
+    meshes = [W.icosphere(3), None, W.icosphere(7), W.icosphere(1), None, W.icosphere(7, amp=0.2), W.icosphere(4)]
+    verts, tris, sizes, base = [], [], [], 0
+    for m in meshes:
+        if m is not None:
+            verts.append(m[0])
+            tris.append(m[1] + base)
+            base += len(m[0])
+        sizes.append(0 if m is None else len(m[1]))
+    verts, tris = np.concatenate(verts), np.concatenate(tris).astype(np.int32)
+    cuts = np.sort(rng.integers(0, nq, len(meshes) - 1))
+    off, qoff = np.concatenate([[0], np.cumsum(sizes)]), np.concatenate([[0], cuts, [nq]])
+    qs = W.uniform_points(nq, 11, -1.5, 1.5)
+    qs[::2] /= np.linalg.norm(qs[::2], axis=1, keepdims=True)  # half of them near the surfaces
+    tv, tt, tq = _cuda(verts), _cuda(tris), _cuda(qs)
+    batch = bq.Batch(bq.triangles.boxes(tt, tv), _cuda(off))
+    for r in (float("inf"), 0.02):
+        many = bq.batched_tri_closest(batch, tt, tv, tq, _cuda(qoff), maxSqrDist=r)
+        few = []
+        for a in range(0, nq, 30_000):
+            part = np.clip(qoff - a, 0, min(30_000, nq - a))
+            few.append(bq.batched_tri_closest(batch, tt, tv, tq[a:a + 30_000], _cuda(part), maxSqrDist=r))
+        assert _same([torch.cat(x) for x in zip(*few)], many), f"radius {r}"
+    ids, d = (x.cpu().numpy() for x in bq.batched_tri_closest(batch, tt, tv, tq, _cuda(qoff))[:2])
+    for s, n in enumerate(sizes):
+        assert (ids[qoff[s]:qoff[s + 1]] >= 0).all() == (n > 0) or qoff[s] == qoff[s + 1]
+        if n:
+            at = rng.integers(qoff[s], qoff[s + 1], 20) if qoff[s] < qoff[s + 1] else []
+            for i in at:
+                assert off[s] <= ids[i] < off[s + 1]
+            d64, _ = oracle.tri_brute_f64(tris[off[s]:off[s + 1]], verts, qs[at])
+            # within the distance's rounding: 2^-20 of the coordinates at hand
+            assert np.all(np.abs(np.sqrt(d[at].astype(np.float64)) - np.sqrt(d64)) <= 2.0 ** -20 * 3)
 
 
 def _limited_allocator(bq, limit):
