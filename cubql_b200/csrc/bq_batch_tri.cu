@@ -251,7 +251,7 @@ int batched_tri_closest(const bq_bvh3f *bvhs, const uint32_t *triOff, const int3
       cudaGetLastError();
     }
     const TriMesh m{nullptr, nullptr, bvhs, triOff, qoff, numSegs, nullptr, tris, verts};
-    launch_tri_group(m, 0, queries, order, nq, maxSqr, ids, d, P, heavy, ovfList, ctl, ctl + 2, ctl + 3, al.s);
+    launch_tri_group(m, 0, queries, order, nq, maxSqr, ids, d, P, heavy, ovfList, ctl, ctl + 2, ctl + 3, nullptr, al.s);
     ProfScope ps("tri.deep", al.s);
     launch_pdl(k_btri_deep<TIE_LOWEST>, dim3(DEEP_THREADS / 128), dim3(128), 0, al.s, bvhs, triOff, qoff, numSegs, tris,
                verts, queries, maxSqr, ids, d, P, ovfList, ctl, deep, err);

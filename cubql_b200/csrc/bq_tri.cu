@@ -307,6 +307,11 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
     heavy = keys[sel];  // the sorted keys are of no further use
   }
   const int b = c.blockSize;
+  auto status_of = [](uint32_t herr) -> int {
+    if (herr & DEV_ERR_STACK) return set_error(BQ_ERR_STACK_OVERFLOW, "query exceeded the deep fallback stack");
+    if (herr & DEV_ERR_TIMEOUT) return set_error(BQ_ERR_TIMEOUT, "query reordering sort timed out");
+    return BQ_OK;
+  };
 #define BQ_TRI_LAUNCH(TIE, ST)                                                                                     \
   ProfScope ps("tri.closest", al.s, 2);                                                                            \
   k_tri<TIE, ST><<<div_up(nq, b), b, TRI_SMEM_STACK * sizeof(StackEntry) * b, al.s>>>(                           \
@@ -319,38 +324,47 @@ int tri_closest(const bq_bvh3f *bvh, const int32_t *tris, const float *verts, co
     else if (c.stackDepth == 64) { BQ_TRI_LAUNCH(TIE_REFERENCE, 64); }
     else { BQ_TRI_LAUNCH(TIE_REFERENCE, 128); }
   } else {
-    float4 *packed = nullptr;
     if (!heavy && tmp.get(&heavy, nq) != BQ_OK) {
       heavy = nullptr;
       cudaGetLastError();
     }
     // a query tests some twenty triangles: the copy pays from about a
     // twentieth as many queries as triangles
-    if ((uint64_t)nq * 16 >= bvh->numPrims) {
+    float4 *packed = nullptr;
+    if (bvh->numPrims && (uint64_t)nq * 16 >= bvh->numPrims) {
       if (tmp.get(&packed, 3ull * bvh->numPrims) != BQ_OK) {
         packed = nullptr;  // no room for the copy: corners through the index
         cudaGetLastError();
       } else {
         ProfScope ps("tri.pack", al.s);
-        launch_pdl(k_tri_pack, dim3(div_up(bvh->numPrims, 256)), dim3(256), 0, al.s, bvh->primIDs, bvh->numPrims, tris,
-                   verts, packed);
+        launch_pdl(k_tri_pack, dim3(div_up(bvh->numNodes, 256)), dim3(256), 0, al.s, nodes, bvh->numNodes, bvh->primIDs,
+                   bvh->numPrims, tris, verts, packed, err);
       }
     }
-    const TriMesh m{nodes, bvh->primIDs, nullptr, nullptr, nullptr, 0, packed, tris, verts};
-    launch_tri_group(m, bvh->numPrims, queries, order, nq, maxSqr, ids, d, P, heavy, ovfList, ovfCount, ovfCount + 2, ovfCount + 3,
-                     al.s);
-    ProfScope ps("tri.deep", al.s);
-    launch_pdl(k_tri_deep<TIE_LOWEST>, dim3(DEEP_THREADS / 128), dim3(128), 0, al.s, nodes, bvh->primIDs, tris, verts,
-               queries, maxSqr, ids, d, P, ovfList, ovfCount, deep, err);
+    auto search = [&](const float4 *corners) {
+      const TriMesh m{nodes, bvh->primIDs, nullptr, nullptr, nullptr, 0, corners, tris, verts};
+      launch_tri_group(m, bvh->numPrims, queries, order, nq, maxSqr, ids, d, P, heavy, ovfList, ovfCount, ovfCount + 2,
+                       ovfCount + 3, corners ? err : nullptr, al.s);
+      ProfScope ps("tri.deep", al.s);
+      launch_pdl(k_tri_deep<TIE_LOWEST>, dim3(DEEP_THREADS / 128), dim3(128), 0, al.s, nodes, bvh->primIDs, tris, verts,
+                 queries, maxSqr, ids, d, P, ovfList, ovfCount, deep, err);
+    };
+    search(packed);
+    uint32_t herr = 0;
+    BQ_CUDA(cudaGetLastError());
+    BQ_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, al.s));
+    BQ_CUDA(cudaStreamSynchronize(al.s));
+    if (!(herr & DEV_ERR_RANGE)) return status_of(herr);
+    // the tree has leaves past the number of prims it was given with
+    BQ_CUDA(cudaMemsetAsync(ovfCount, 0, 16, al.s));
+    search(nullptr);
   }
 #undef BQ_TRI_LAUNCH
   BQ_CUDA(cudaGetLastError());
   uint32_t herr = 0;
   BQ_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, al.s));
   BQ_CUDA(cudaStreamSynchronize(al.s));
-  if (herr & DEV_ERR_STACK) return set_error(BQ_ERR_STACK_OVERFLOW, "query exceeded the deep fallback stack");
-  if (herr & DEV_ERR_TIMEOUT) return set_error(BQ_ERR_TIMEOUT, "query reordering sort timed out");
-  return BQ_OK;
+  return status_of(herr);
 }
 
 int tri_distance_bwd(const int32_t *tris, const float *verts, uint32_t numVerts, const float *queries, uint32_t nq,

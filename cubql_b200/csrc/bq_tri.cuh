@@ -539,9 +539,10 @@ constexpr uint32_t TRI_ALL = 0xffffffffu;
 __global__ void __launch_bounds__(128) k_tri_near(TriMesh m, const float *__restrict__ queries,
                                                   const uint32_t *__restrict__ order, uint32_t nq, uint32_t rounds,
                                                   float maxSqr, int32_t *outIds, float *outD, float *outP,
-                                                  uint32_t *leftList, uint32_t *leftCount)
+                                                  uint32_t *leftList, uint32_t *leftCount, const uint32_t *stop)
 {
   griddep_wait();
+  if (stop && (*stop & DEV_ERR_RANGE)) return;
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, tt = min(t, nq - 1);
   const uint32_t qi = order ? __ldg(order + tt) : tt;
   const float *p = queries + 3ull * qi;
@@ -597,9 +598,10 @@ __global__ void __launch_bounds__(128, 8) k_tri_left(TriMesh m, const float *__r
 __global__ void __launch_bounds__(128, 8) k_tri_group(TriMesh m, const float *__restrict__ queries,
                                                    const uint32_t *__restrict__ order, uint32_t nq, uint32_t run,
                                                    float maxSqr, int32_t *outIds, float *outD, float *outP,
-                                                   uint32_t *leftList, uint32_t *leftCount)
+                                                   uint32_t *leftList, uint32_t *leftCount, const uint32_t *stop)
 {
   griddep_wait();
+  if (stop && (*stop & DEV_ERR_RANGE)) return;
   __shared__ TriGroupShared<TRI_GROUP, TRI_GROUP_STACK> sh[128 / TRI_GROUP];
   const uint32_t g = threadIdx.x / TRI_GROUP;
   const uint64_t at = ((uint64_t)blockIdx.x * (128 / TRI_GROUP) + g) * run;
@@ -624,13 +626,10 @@ __global__ void __launch_bounds__(128) k_tri_heavy(TriMesh m, const float *__res
 // from its neighbour's triangle, while every SM still gets its groups
 inline uint32_t tri_run(uint32_t nq) { return std::min(8u, std::max(1u, nq >> 17)); }
 
-// corners of every triangle in leaf order
-__global__ void k_tri_pack(const uint32_t *__restrict__ primIDs, uint32_t numPrims, const int32_t *__restrict__ tris,
-                           const float *__restrict__ verts, float4 *__restrict__ packed)
+__device__ __forceinline__ void pack_corners(uint32_t j, const uint32_t *__restrict__ primIDs,
+                                             const int32_t *__restrict__ tris, const float *__restrict__ verts,
+                                             float4 *__restrict__ packed)
 {
-  griddep_wait();
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= numPrims) return;
   const uint32_t id = __ldg(primIDs + j);
   const int32_t *t = tris + 3ull * id;
   const V3 a = ldv(verts, __ldg(t)), b = ldv(verts, __ldg(t + 1)), c = ldv(verts, __ldg(t + 2));
@@ -639,26 +638,57 @@ __global__ void k_tri_pack(const uint32_t *__restrict__ primIDs, uint32_t numPri
   packed[3ull * j + 2] = make_float4(c.x, c.y, c.z, 0.f);
 }
 
+// Corners of the triangles in leaf order.  Leaf by leaf, a thread a node: the
+// list of prim ids may go on after the last leaf with prims that have no box,
+// and their index triples need not be usable.  Long leaves are shared by the
+// warp.  A leaf that goes past numPrims sets DEV_ERR_RANGE, and the search that
+// would use the copy does not start (`stop`).
+__global__ void k_tri_pack(const Node *__restrict__ nodes, uint32_t numNodes, const uint32_t *__restrict__ primIDs,
+                           uint32_t numPrims, const int32_t *__restrict__ tris, const float *__restrict__ verts,
+                           float4 *__restrict__ packed, uint32_t *err)
+{
+  griddep_wait();
+  constexpr uint32_t SHORT = 4;
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  uint32_t off = 0, cnt = 0;
+  if (t < numNodes && t != 1) {  // node 1 is unused
+    const uint64_t admin = ldg_admin(nodes + t);
+    off = (uint32_t)admin_offset(admin);
+    cnt = admin_count(admin);
+    if (cnt && (uint64_t)off + cnt > numPrims) {
+      atomicOr(err, DEV_ERR_RANGE);
+      cnt = 0;
+    }
+  }
+  if (cnt <= SHORT)
+    for (uint32_t j = 0; j < cnt; j++) pack_corners(off + j, primIDs, tris, verts, packed);
+  for (uint32_t m = __ballot_sync(0xffffffffu, cnt > SHORT); m; m &= m - 1) {
+    const uint32_t from = __ffs(m) - 1;
+    const uint32_t o = __shfl_sync(0xffffffffu, off, from), n = __shfl_sync(0xffffffffu, cnt, from);
+    for (uint32_t j = lane; j < n; j += 32) pack_corners(o + j, primIDs, tris, verts, packed);
+  }
+}
+
 // The launches; queries that none finished are on ovfList.  numPrims: of the
 // tree (0 for a batch: k_tri_near looks at each).  heavy: a list of nq words, or
 // null when there is no room for one: each query is then answered by a thread.
-// The counts are zeroed.
+// The counts are zeroed.  stop: the word in which k_tri_pack reports, or null.
 inline void launch_tri_group(const TriMesh &m, uint32_t numPrims, const float *queries, const uint32_t *order, uint32_t nq, float maxSqr,
                              int32_t *ids, float *d, float *P, uint32_t *heavy, uint32_t *ovfList, uint32_t *ovfCount,
-                             uint32_t *heavyCount, uint32_t *nearCount, cudaStream_t s)
+                             uint32_t *heavyCount, uint32_t *nearCount, const uint32_t *stop, cudaStream_t s)
 {
   const uint32_t run = tri_run(nq);
   if (!heavy) {
     ProfScope ps("tri.near", s);
     launch_pdl(k_tri_near, dim3(div_up(nq, 128)), dim3(128), 0, s, m, queries, order, nq, TRI_ALL, maxSqr, ids, d, P,
-               ovfList, ovfCount);
+               ovfList, ovfCount, stop);
     return;
   }
   if (nq >= TRI_NEAR_MIN && numPrims <= TRI_NEAR_PRIMS) {
     {
       ProfScope ps("tri.near", s);
       launch_pdl(k_tri_near, dim3(div_up(nq, 128)), dim3(128), 0, s, m, queries, order, nq,
-                 tri_near_rounds(nq), maxSqr, ids, d, P, ovfList, nearCount);
+                 tri_near_rounds(nq), maxSqr, ids, d, P, ovfList, nearCount, stop);
     }
     ProfScope ps("tri.group", s);
     launch_pdl(k_tri_left, dim3(div_up((uint64_t)div_up(nq, run) * TRI_GROUP, 128)), dim3(128), 0, s, m, queries, run,
@@ -666,7 +696,7 @@ inline void launch_tri_group(const TriMesh &m, uint32_t numPrims, const float *q
   } else {
     ProfScope ps("tri.group", s);
     launch_pdl(k_tri_group, dim3(div_up((uint64_t)div_up(nq, run) * TRI_GROUP, 128)), dim3(128), 0, s, m, queries,
-               order, nq, run, maxSqr, ids, d, P, heavy, heavyCount);
+               order, nq, run, maxSqr, ids, d, P, heavy, heavyCount, stop);
   }
   ProfScope ps("tri.heavy", s);
   launch_pdl(k_tri_heavy, dim3(4 * num_sms()), dim3(128), 0, s, m, queries, maxSqr, ids, d, P,

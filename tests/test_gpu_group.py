@@ -218,6 +218,36 @@ def test_triangle_threads_before_groups(bq, n, nq):
         assert _same(few, many), f"radius {r}"
 
 
+@pytest.mark.parametrize("leaf", [1, 40])
+@pytest.mark.parametrize("builder", ["gpuBuilder", "sahBuilder", "radixBuilder"])
+def test_triangles_without_a_box_are_not_read(bq, builder, leaf):
+    """Removed triangles (an empty box, indices that point nowhere) are listed
+    after the others by some builders; a tree handed in need not say how many
+    prims it has.  The corners of neither are copied."""
+    tv, tt = _mesh(4)
+    tq = _cuda(W.uniform_points(3000, 4, -1.5, 1.5))
+    boxes = bq.triangles.boxes(tt, tv)
+    build = bq.gpuBuilder if builder == "gpuBuilder" else getattr(bq.cuda, builder)
+    bvh = build(boxes, bq.BuildConfig(makeLeafThreshold=leaf))
+    want = bq.triangles.findClosest(bvh, tt, tv, tq)
+    n = bvh.c.numPrims
+    for fewer in (n - 7, 1, 0):
+        bvh.c.numPrims = fewer
+        assert _same(bq.triangles.findClosest(bvh, tt, tv, tq), want), fewer
+    bvh.c.numPrims = n
+    bvh.free()
+    gone = torch.rand(len(tt), generator=torch.Generator().manual_seed(1)) < 0.3
+    tt2 = tt.clone()
+    tt2[gone.cuda()] = -(1 << 30)
+    empty = boxes.clone()
+    empty[gone.cuda()] = torch.tensor([np.inf] * 3 + [-np.inf] * 3, device="cuda", dtype=torch.float32)
+    bvh = build(empty, bq.BuildConfig(makeLeafThreshold=leaf))
+    kept = build(boxes[~gone.cuda()].contiguous(), bq.BuildConfig(makeLeafThreshold=leaf))
+    ids, d, p = bq.triangles.findClosest(bvh, tt2, tv, tq)
+    wi, wd, wp = bq.triangles.findClosest(kept, tt[~gone.cuda()].contiguous(), tv, tq)
+    assert _same((d, p), (wd, wp)) and torch.equal(ids.cpu(), torch.nonzero(~gone)[:, 0].int()[wi.cpu().long()])
+
+
 @pytest.mark.parametrize("nq", [300_000, 1_100_000])
 def test_batched_triangles_sorted_and_seeded(bq, oracle, nq):
     """Meshes too large for a thread a query (its groups start from their
