@@ -44,18 +44,24 @@ constexpr int KNN_SMEM_STACK = 0;
 // 0.323 0.353).  Once the nodes are far larger than L2 the order pays sooner:
 // 5M points, leaves of one (320 MB) 131,100 0.235 and 0.222, 200,000 0.255 and
 // 0.270; 7M 0.241 0.246; 10M (640 MB) 0.245 0.267, and 100,000 equal at 0.233.
+// Clustered queries gain more from the order: 2M points of the 64-Gaussian
+// mixture, reference's rule, 100,000 0.170 and 0.161, 200,000 0.191 0.216,
+// 250,000 0.205 0.237 (leaves of eight 0.192 0.176, 0.193 0.225, 0.207 0.318).
+// The line lies between the two.
 // kNN, k = 8: 1,001 0.149 and 0.124, 5,003 0.172 and 0.161, 16,001 equal,
 // 50,001 0.205 and 0.313; the shared search needs the order, and with long
 // lists it pays from the start (k = 32, 1,001: 0.195 and 0.259).
 inline bool cp_order_pays(uint32_t nq, uint32_t numNodes)
 {
-  return nq >= (1u << 18) || (nq >= (1u << 16) && (uint64_t)nq * numNodes >= 1700000000000ull);
+  return nq >= (3u << 16) || (nq >= (1u << 16) && (uint64_t)nq * numNodes >= 1700000000000ull);
 }
 inline uint32_t knn_order_min(int k) { return k <= 8 ? 4096 : 2; }
 // Longest lists whose searches, a thread each, do not walk in step: inserting
 // into them costs little, so leaves are better taken at once (2M points and
 // queries, plain and in step, ms: k = 1 1.01 and 1.26, 4 1.84 and 1.99, 5 2.31
-// and 2.47, 8 3.09 and 3.01, 16 6.75 and 5.08).
+// and 2.47, 8 3.09 and 3.01, 16 6.75 and 5.08).  Leaves of several prims cost
+// more (400,000 points, leaves of eight, 2,000 queries, k = 4: 0.201 and
+// 0.177).
 constexpr int KNN_PLAIN_MAX = 5;
 
 // rootBox: lower xyz, upper xyz (the first 24 bytes of a binary root node)
@@ -247,7 +253,8 @@ __global__ void __launch_bounds__(128) k_knn(const Node *__restrict__ nodes, con
   const uint32_t qi = order ? __ldg(order + min(t, nq - 1)) : min(t, nq - 1);
   extern __shared__ StackEntry sStack[];
   HybridStack<KNN_SMEM_STACK, STACK> st(sStack);
-  if (!run_knn<K, TIE, STEP>(alive, nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD, numFound))
+  if (!run_knn<K, TIE, STEP>(alive, nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD,
+                             numFound))
     ovfList[atomicAdd(ovfCount, 1u)] = qi;
 }
 
@@ -263,7 +270,8 @@ __global__ void k_knn_deep(const Node *__restrict__ nodes, const uint32_t *__res
   for (uint32_t w = tid; w < cnt; w += gridDim.x * blockDim.x) {
     const uint32_t qi = ovfList[w];
     GlobalStack st{stacks + (size_t)tid * DEEP_STACK, DEEP_STACK, 0};
-    if (!run_knn<K, TIE, false>(true, nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD, numFound)) {
+    if (!run_knn<K, TIE, false>(true, nodes, primIDs, points, queries, qi, k, maxSqr, maxSqr, st, outIds, outD,
+                                numFound)) {
       for (int j = 0; j < k; j++) {
         outIds[(size_t)qi * k + j] = -1;
         outD[(size_t)qi * k + j] = INFINITY;
@@ -446,8 +454,9 @@ void launch_cp(const bq_bvh3f *bvh, const float *points, const float *queries, u
     // to 8, 2.8 prims a node: 0.581 -> 0.549 ms), short ones are not (up to
     // 4, 1.3 a node: 0.522 -> 0.560; leaves of one: 3.8 -> 4.9).
     const bool step = bvh->numPrims / 2 >= bvh->numNodes;
-    launch_pdl(step ? k_closest<TIE, STACK, true> : k_closest<TIE, STACK, false>, dim3(div_up(nq, block)), dim3(block), SMEM_STACK * sizeof(StackEntry) * block,
-               s, nodes, bvh->primIDs, points, queries, qs.order, nq, maxSqr, ids, d, qs.ovfList, qs.ovfCount, ex);
+    launch_pdl(step ? k_closest<TIE, STACK, true> : k_closest<TIE, STACK, false>, dim3(div_up(nq, block)), dim3(block),
+               SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries, qs.order, nq, maxSqr,
+               ids, d, qs.ovfList, qs.ovfCount, ex);
   }
   ProfScope ps("query.deep", s);
   launch_pdl(k_closest_deep<TIE>, dim3(DEEP_THREADS / 128), dim3(128), 0, s, nodes, bvh->primIDs, points, queries,
@@ -475,9 +484,10 @@ void launch_knn(const bq_bvh3f *bvh, const float *points, const float *queries, 
                qs.ovfCount);
   } else {
     ProfScope ps("query.knn", s);
-    launch_pdl(k > KNN_PLAIN_MAX ? k_knn<K, TIE, STACK, (K > 4)> : k_knn<K, TIE, STACK, (K > 8)>, dim3(div_up(nq, block)),
-               dim3(block), KNN_SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries,
-               qs.order, nq, k, maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);
+    const bool step = k > KNN_PLAIN_MAX || bvh->numPrims / 2 >= bvh->numNodes;
+    launch_pdl(step ? k_knn<K, TIE, STACK, true> : k_knn<K, TIE, STACK, (K > 8)>, dim3(div_up(nq, block)), dim3(block),
+               KNN_SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries, qs.order, nq, k, maxSqr,
+               ids, d, nf, qs.ovfList, qs.ovfCount);
   }
   ProfScope ps("query.deep", s);
   launch_pdl(k_knn_deep<K, TIE>, dim3(DEEP_THREADS / 128), dim3(128), 0, s, nodes, bvh->primIDs, points, queries, k,

@@ -65,6 +65,22 @@ def test_knn_where_the_shared_search_begins(bq, n, nq, k, shared):
     bvh.free()
 
 
+@pytest.mark.parametrize("tie", [0, 1])
+@pytest.mark.parametrize("k", [1, 4, 5, 6])
+@pytest.mark.parametrize("leaf", [1, 8])
+def test_knn_plain_and_in_step_match_oracle(bq, oracle, tie, k, leaf):
+    """A thread a query, on its own (short lists over short leaves) and with
+    the warp in step."""
+    pts, qs = W.uniform_points(5000), W.uniform_points(333, 5, -0.1, 1.1)
+    bvh = bq.cuda.radixBuilder(_cuda(boxes_np(pts)), bq.BuildConfig(makeLeafThreshold=leaf))
+    assert (bvh.numPrims // 2 >= bvh.numNodes) == (leaf == 8)
+    n, pr = bvh.to_host()
+    want = oracle.knn(n, pr, pts, qs, k, tie_mode=tie)
+    got = bq.points.findKNN(bvh, _cuda(pts), _cuda(qs), k, qcfg=bq.query_config(tieMode=tie))
+    for a, b in zip(got, want):
+        assert np.array_equal(a.cpu().numpy(), b)
+
+
 def test_knn_shared_search_on_duplicates_and_clusters(bq):
     """Copies of points (ids decide); tight clusters, planes and lines that
     the queries are far from, and queries far outside: their warps give the
@@ -375,20 +391,20 @@ def test_closest_point_where_sorting_begins(bq, tie, leaf):
     that are processed at once and in step."""
     pts = W.uniform_points(30000)
     tp = _cuda(pts)
-    qs = _cuda(W.uniform_points(262145, W.SEED_QUERIES, -0.1, 1.1))
+    qs = _cuda(W.uniform_points(196609, W.SEED_QUERIES, -0.1, 1.1))
     bvh = bq.gpuBuilder(_cuda(boxes_np(pts)), bq.BuildConfig(makeLeafThreshold=leaf))
     b = bq.points.findClosest(bvh, tp, qs, qcfg=bq.query_config(tieMode=tie, reorder=0))
-    for nq in (1, 33, 262143, 262144, 262145):
+    for nq in (1, 33, 196607, 196608, 196609):
         a, ran = _phases(bq, lambda: bq.points.findClosest(bvh, tp, qs[:nq], qcfg=bq.query_config(tieMode=tie)))
-        assert _same(a, [x[:nq] for x in b]) and ("query.keys" in ran) == (nq >= 262144), nq
+        assert _same(a, [x[:nq] for x in b]) and ("query.keys" in ran) == (nq >= 196608), nq
 
 
 def test_closest_point_over_many_nodes_is_sorted_sooner(bq):
     g = torch.Generator(device="cuda").manual_seed(2)
-    tp = torch.rand((4_000_000, 3), generator=g, device="cuda")
+    tp = torch.rand((5_000_000, 3), generator=g, device="cuda")
     bvh = bq.cuda.radixBuilder(bq.points_to_boxes(tp))
     first = -(-1_700_000_000_000 // bvh.numNodes)
-    assert 1 << 16 < first < 1 << 18
+    assert 1 << 16 < first < 3 << 16
     qs = torch.rand((first, 3), generator=g, device="cuda")
     b = bq.points.findClosest(bvh, tp, qs, qcfg=bq.query_config(reorder=0))
     for nq in (first - 1, first):
