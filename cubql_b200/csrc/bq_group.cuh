@@ -13,8 +13,11 @@
 // down the tree (25 of them before every lane has k prims), 481 prims
 // tested, 64 of them wanted by a lane, 8 merges.  One thread per query had 5
 // of 32 lanes active and 76,000 instructions a warp, waiting on dependent
-// loads: 32.7 ms; this takes 15.0 ms, bound by issue slots and the L1 data
-// pipe (67% of its wavefronts).  What made the difference, ms: inserting
+// loads: 32.7 ms, 25 with the warp's traversals in step; this takes 15.2 ms
+// with 30 lanes active.  Of 2M over 2M (3.2 ms): issue slots 51% busy, L1 data
+// pipe 56% of its wavefronts, 17 warps an SM (shared memory and registers)
+// that wait on loads and on the list code, whose 16 keys lie in local memory.
+// What made the difference, ms: inserting
 // each prim into the sorted list as it is met 53, merging 16 at a time 15.7,
 // registers capped for five blocks an SM 15.0.  The Hilbert order instead of
 // Morton: 2M points, 1M queries, k = 32: 10.9 -> 5.2 before the merges, as a
@@ -298,8 +301,8 @@ __device__ __forceinline__ bool group_radius_pays(const Node *nodes, uint32_t nu
 
 // Blocks of 128 threads for the queries that the shared search has left: one
 // for every 128 queries of the call, though most find nothing, as those left
-// take very different times.  512 clouds: 62 ms with 8 an SM that go through
-// the list, 59 with 64, 57.5 so.
+// take very different times.  512 clouds: 58.9 ms with 64 blocks an SM that go
+// through the list, 57.5 so.
 inline int knn_left_blocks(uint32_t nq) { return div_up(nq, 128); }
 
 // whether a query can take part: it is finite and its distance to the tree

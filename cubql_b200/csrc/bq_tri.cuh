@@ -19,13 +19,14 @@
 // query, the warps in step, for some rounds; the groups get what is left, each
 // query with the triangle found so far (figures at TRI_NEAR_PRIMS).
 //
-// 4M queries over 1.31M triangles: 50-57 ms with one thread per query (the
-// last warps ran alone for 20 ms), 22.8 ms so: 20.5 for the first launch,
-// bound by the L1 data pipe (89% of its wavefronts), 2.3 for the second.
+// 4M queries over 1.31M triangles: 46-50 ms with one thread per query (the
+// last warps ran alone for 20 ms), 23.0 so: 20.9 for the first launch, bound by
+// the L1 data pipe (90% of its wavefronts), 2.1 for the second.
 // Four lanes a query 23.5 ms, sixteen 32.9; one lane a child instead of a
 // pair of children 19.1 + 4.7 ms.  5,001 queries over the same mesh: 14.5
-// -> 0.9 ms.  A batch of 128 meshes, 6.4M queries: 19.3 -> 14.6 ms, of which
-// sorting the queries, which it did not do before, takes 0.6.
+// -> 0.9 ms.  A batch of 128 meshes, 6.4M queries: 19.3 -> 14.6 ms by groups
+// alone, 11.8 with threads first (sorting the queries, which it did not do
+// before, takes 0.6 of it).
 //
 // The answer, the lowest id among equal distances, is a function of the query
 // and the triangles alone, not of the tree, the batch or the visiting order

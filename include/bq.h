@@ -111,17 +111,22 @@ typedef struct bq_allocator {
   int scratchFromPool;
 } bq_allocator;
 
-/* traversal knobs; NULL = defaults (ties lowest-ID, Morton-ordered
-   queries, autotuned launch shape) */
+/* traversal knobs; NULL = defaults (ties lowest-ID, large batches ordered
+   along a space-filling curve, 64 stack entries, 128 threads a block) */
 typedef struct bq_query_config {
   int tieMode;       /* BQ_TIES_LOWEST_ID or BQ_TIES_REFERENCE */
-  int stackDepth;    /* fast-path stack entries: 32, 64 or 128 (0 = 64) */
-  int blockSize;     /* threads per block: 64..512 (0 = 128) */
+  int stackDepth;    /* stack entries of a thread's traversal: 32, 64 or 128 (0 = 64).  The searches
+                        that lanes share (kNN and triangles, lowest-id ties) have stacks of
+                        their own. */
+  int blockSize;     /* threads per block: 64 or 128 (0 = 128) */
   int reorder;       /* 1 = process queries along a space-filling curve (small batches: as given), 0 = as given */
-  int queriesPerWarp;/* one thread per query; queries a warp takes per work grab in the
-                        persistent batched kernel (multiple of 32, <= 1024; 0 = 32) */
-  int lanesPerQuery; /* bq_knn_f3 only.  0 or 1: one thread per query, its top-k list in
-                        that thread's registers.  4, 8, 16 or 32 (at least k): a group of
+  int queriesPerWarp;/* queries a warp takes per work grab where bq_batched_knn_f3 runs its
+                        persistent kernel: k below 5 or above 32, the reference's ties, or
+                        reorder 0 (multiple of 32, <= 1024; 0 = 32) */
+  int lanesPerQuery; /* bq_knn_f3 only.  0 or 1: each query's top-k list in one thread's
+                        registers, searched for by that thread or, with lowest-id ties, k <= 32
+                        and enough queries among the prims, by one search for a warp's 32
+                        queries.  4, 8, 16 or 32 (at least k): a group of
                         that many lanes per query walks the tree together and holds the
                         sorted top-k list one candidate per lane; a new candidate is
                         placed by one ballot and moved in by one warp shuffle */
@@ -450,10 +455,12 @@ int bq_batched_build_morton63_f3(const bq_box3f *boxes, const uint32_t *segOffse
 /* k nearest points per query over a batch built by the call above.
    Queries are stored cloud by cloud (queryOffsets: device, numSegs+1
    entries); query q of cloud s searches only cloud s (whose points start
-   at points + 3*pointOffsets[s]).  ids are cloud-local.  A persistent
-   work-stealing kernel answers the whole batch; qcfg->queriesPerWarp
-   (a multiple of 32, default 32) is the number of queries a warp takes
-   per grab.  No host synchronisation. */
+   at points + 3*pointOffsets[s]).  ids are cloud-local.  With lowest-id
+   ties and k of 5 to 32 a warp makes one search for its 32 queries where a
+   cloud has enough of them, and a second launch answers the rest a thread
+   each; otherwise a persistent kernel takes qcfg->queriesPerWarp queries
+   (a multiple of 32, default 32) per warp and grab.  No host
+   synchronisation. */
 int bq_batched_knn_f3(const bq_bvh3f *bvhs, const uint32_t *pointOffsets, const float *points, const float *queries,
                       const uint32_t *queryOffsets, uint32_t numSegs, uint32_t numQueries, int k, float maxSqrDist,
                       const bq_query_config *qcfg, int32_t *ids, float *sqrDist, int32_t *numFound,
