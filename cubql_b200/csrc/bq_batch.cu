@@ -524,8 +524,8 @@ int launch_seg_knn(const bq_bvh3f *bvhs, const uint32_t *poff, const float *poin
                  skeys, order, nq, k, maxSqr, ids, d, nf, leftList, workCtr);
     }
     ProfScope ps("batch.knn_left", s);
-    launch_pdl(k_seg_knn_left<KK, STACK>, dim3(knn_left_blocks(nq)), dim3(128), 0, s, bvhs, poff, points, queries, skeys,
-               order, (const uint32_t *)leftList, (const uint32_t *)workCtr, k, maxSqr, ids, d, nf, ovfList, ovfCount);
+    launch_pdl(k_seg_knn_left<KK, STACK>, dim3(knn_left_blocks(nq)), dim3(128), 0, s, bvhs, poff, points, queries,
+               skeys, order, (const uint32_t *)leftList, (const uint32_t *)workCtr, k, maxSqr, ids, d, nf, ovfList, ovfCount);
   } else {
     int perSm = 0;
     BQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_seg_knn<K, TIE, STACK>, block, 0));
@@ -706,7 +706,7 @@ int batched_knn(const bq_bvh3f *bvhs, const uint32_t *poff, const float *points,
 #define BQ_SEG_KNN(KK)                                                                                             \
   (tie == BQ_TIES_REFERENCE                                                                                        \
        ? stack_dispatch<KK, TIE_REFERENCE>(st, bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, b, \
-                                           chunk, ctl, ids, d, nf, ovfList, ctl + 1, deep, leftList, dErr, al.s)                    \
+                                           chunk, ctl, ids, d, nf, ovfList, ctl + 1, deep, leftList, dErr, al.s)   \
        : stack_dispatch<KK, TIE_LOWEST>(st, bvhs, poff, points, queries, qoff, skeys, order, nq, k, maxSqr, b,    \
                                         chunk, ctl, ids, d, nf, ovfList, ctl + 1, deep, leftList, dErr, al.s))
   int s;

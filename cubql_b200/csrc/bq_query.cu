@@ -30,9 +30,9 @@ namespace {
 // stack entries a closest-point thread keeps in shared memory (the top of
 // its traversal stack); the rest of the stack is in local memory.  8 took
 // 10M closest-point queries from 4.17 to 3.69 ms (4: 3.92, 12: 3.83, 16:
-// 3.99).  The kNN kernel, at 62 registers and fewer threads per SM, gained
-// nothing from it (29.7 ms with none, 29.8-30.3 with 4..16), so its stack
-// stays in local memory.
+// 3.99).  kNN with a thread a query, at 62 registers and fewer threads per SM,
+// gained nothing from it (before its warps walked in step: 29.7 ms with none,
+// 29.8-30.3 with 4..16), so its stack stays in local memory.
 constexpr int SMEM_STACK = 8;
 constexpr int KNN_SMEM_STACK = 0;
 
@@ -193,7 +193,8 @@ __device__ __forceinline__ bool run_knn(bool alive, const Node *nodes, const uin
 template <int K>
 __global__ void __launch_bounds__(128, GroupShape<K>::BLOCKS)
     k_knn_warp(const Node *__restrict__ nodes, uint32_t numPrims, const uint32_t *__restrict__ primIDs,
-               const float *__restrict__ points, const float *__restrict__ queries, const uint32_t *__restrict__ order, uint32_t nq, int k, float maxSqr,
+               const float *__restrict__ points, const float *__restrict__ queries,
+               const uint32_t *__restrict__ order, uint32_t nq, int k, float maxSqr,
                int32_t *__restrict__ outIds, float *__restrict__ outD, int32_t *__restrict__ numFound,
                uint32_t *__restrict__ leftList, uint32_t *leftCount)
 {
@@ -486,8 +487,8 @@ void launch_knn(const bq_bvh3f *bvh, const float *points, const float *queries, 
     ProfScope ps("query.knn", s);
     const bool step = k > KNN_PLAIN_MAX || bvh->numPrims / 2 >= bvh->numNodes;
     launch_pdl(step ? k_knn<K, TIE, STACK, true> : k_knn<K, TIE, STACK, (K > 8)>, dim3(div_up(nq, block)), dim3(block),
-               KNN_SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries, qs.order, nq, k, maxSqr,
-               ids, d, nf, qs.ovfList, qs.ovfCount);
+               KNN_SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries, qs.order, nq, k,
+               maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);
   }
   ProfScope ps("query.deep", s);
   launch_pdl(k_knn_deep<K, TIE>, dim3(DEEP_THREADS / 128), dim3(128), 0, s, nodes, bvh->primIDs, points, queries, k,
@@ -588,8 +589,8 @@ __global__ void k_fill_empty(uint32_t nq, int k, int32_t *ids, float *d, int32_t
 void query_keys(const float *rootBox, const float *queries, uint32_t nq, bool hilbert, uint32_t *keys, uint32_t *idx,
                 cudaStream_t s)
 {
-  launch_pdl(hilbert ? k_query_keys<true> : k_query_keys<false>, dim3(div_up(nq, 256)), dim3(256), 0, s, rootBox, queries,
-             nq, keys, idx);
+  launch_pdl(hilbert ? k_query_keys<true> : k_query_keys<false>, dim3(div_up(nq, 256)), dim3(256), 0, s, rootBox,
+             queries, nq, keys, idx);
 }
 
 int prepare_queries(const float *rootBox, const float *queries, uint32_t nq, bool reorder, bool hilbert, TempSet &tmp,
@@ -670,8 +671,8 @@ int closest_point(const bq_bvh3f *bvh, const float *points, const float *queries
   }
   TempSet tmp(al);
   QueryScratch qs;
-  BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0 && cp_order_pays(nq, bvh->numNodes), false,
-                         tmp, al, qs));
+  BQ_TRY(prepare_queries((const float *)bvh->nodes, queries, nq, c.reorder != 0 && cp_order_pays(nq, bvh->numNodes),
+                         false, tmp, al, qs));
   const int tie = c.tieMode, st = c.stackDepth, b = c.blockSize;
   if (tie == BQ_TIES_REFERENCE) {
     if (st == 32) launch_cp<TIE_REFERENCE, 32>(bvh, points, queries, nq, maxSqr, b, ids, d, qs, al.s, ex);

@@ -194,8 +194,10 @@ __device__ __forceinline__ bool push_child(Stack &stack, uint32_t idx, uint64_t 
 // at an inner node open it or, once as many lanes wait at a leaf, all of
 // those process their leaf.  A leaf that costs much (kNN inserts into its
 // list) is then paid for by many lanes at once: 10M kNN16 queries 32.7 ->
-// 25.4 ms (13 of 32 lanes active instead of 5), 1M under the reference's
-// rule 1.17 -> 1.12 ms; waiting for twice or half as many lanes 26.3, 25.8.
+// 25.4 ms (13 of 32 lanes active instead of 5); waiting for twice or half as
+// many lanes 26.3, 25.8.  Where neighbours want the same leaves it costs
+// something: 10M queries over 10M points of a mixture with many copies, the
+// reference's rule, 5.5 -> 5.9.
 // A cheap leaf is better taken at once (closest point over leaves of one
 // prim 3.8 -> 4.9 ms).
 // LIMITED: lanes that are not done after `rounds` rounds return false.

@@ -674,9 +674,10 @@ __global__ void k_tri_pack(const Node *__restrict__ nodes, uint32_t numNodes, co
 // tree (0 for a batch: k_tri_near looks at each).  heavy: a list of nq words, or
 // null when there is no room for one: each query is then answered by a thread.
 // The counts are zeroed.  stop: the word in which k_tri_pack reports, or null.
-inline void launch_tri_group(const TriMesh &m, uint32_t numPrims, const float *queries, const uint32_t *order, uint32_t nq, float maxSqr,
-                             int32_t *ids, float *d, float *P, uint32_t *heavy, uint32_t *ovfList, uint32_t *ovfCount,
-                             uint32_t *heavyCount, uint32_t *nearCount, const uint32_t *stop, cudaStream_t s)
+inline void launch_tri_group(const TriMesh &m, uint32_t numPrims, const float *queries, const uint32_t *order,
+                             uint32_t nq, float maxSqr, int32_t *ids, float *d, float *P, uint32_t *heavy,
+                             uint32_t *ovfList, uint32_t *ovfCount, uint32_t *heavyCount, uint32_t *nearCount,
+                             const uint32_t *stop, cudaStream_t s)
 {
   const uint32_t run = tri_run(nq);
   if (!heavy) {

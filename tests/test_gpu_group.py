@@ -88,7 +88,8 @@ def test_knn_shared_search_on_duplicates_and_clusters(bq):
     rng = np.random.default_rng(3)
     u = W.uniform_points(20000, 9)
     dup = np.repeat(W.uniform_points(300), 40, axis=0)
-    clu = (W.uniform_points(8, 5)[rng.integers(0, 8, 20000)] + 0.002 * rng.standard_normal((20000, 3))).astype(np.float32)
+    clu = W.uniform_points(8, 5)[rng.integers(0, 8, 20000)]
+    clu = (clu + 0.002 * rng.standard_normal((20000, 3))).astype(np.float32)
     for pts, qs in ((dup, np.concatenate([dup[::2], W.uniform_points(9000, 9)])), (clu, u),
                     (u * np.float32([1, 1, 0]), u), (u * np.float32([1, 0, 0]), u), (u, 3 * u - 1),
                     (np.repeat(u[:1], 40, axis=0), u)):
@@ -204,7 +205,8 @@ def test_triangle_slivers_do_not_depend_on_batch_or_tree(bq):
     rng = np.random.default_rng(9)
     c = rng.uniform(-1, 1, (3000, 1, 3))
     e = rng.standard_normal((3000, 1, 3)) * 0.3
-    v = c + e * np.array([0.0, 0.5, 1.0])[None, :, None] + rng.standard_normal((3000, 3, 3)) * 10.0 ** rng.uniform(-8, -2, (3000, 1, 1))
+    v = c + e * np.array([0.0, 0.5, 1.0])[None, :, None]  # three points on a line, moved by 1e-8 to 1e-2
+    v += rng.standard_normal((3000, 3, 3)) * 10.0 ** rng.uniform(-8, -2, (3000, 1, 1))
     verts, tris = v.reshape(-1, 3).astype(np.float32), np.arange(9000, dtype=np.int32).reshape(-1, 3)
     tv, tt, tq = _cuda(verts), _cuda(tris), _cuda(_near_queries(verts, tris, 400_000, rng))
     boxes = bq.triangles.boxes(tt, tv)
@@ -230,7 +232,8 @@ def test_triangle_threads_before_groups(bq, n, nq):
     tq, bvh = _cuda(qs), bq.cuda.radixBuilder(bq.triangles.boxes(tt, tv))
     for r in (float("inf"), 0.01):
         many = bq.triangles.findClosest(bvh, tt, tv, tq, maxSqrDist=r)
-        few = [torch.cat(x) for x in zip(*[bq.triangles.findClosest(bvh, tt, tv, q, maxSqrDist=r) for q in tq.split(30_000)])]
+        few = [bq.triangles.findClosest(bvh, tt, tv, q, maxSqrDist=r) for q in tq.split(30_000)]
+        few = [torch.cat(x) for x in zip(*few)]
         assert _same(few, many), f"radius {r}"
 
 
