@@ -278,12 +278,14 @@ __device__ __forceinline__ bool group_search(const Node *__restrict__ nodes, con
 // and 5.08; k = 32 at 1/4 2.88 and 3.21, at 1/2 3.78 and 5.77.  200,000
 // points: k = 16 at 1/2 0.52 and 0.41, at 1 0.48 and 0.66.  20,000: k = 8 at 1
 // 0.22 and 0.20, at 2 0.16 and 0.21; k = 16 at 1/2 0.37 and 0.24 (too few
-// warps to hide the steps).
+// warps to hide the steps).  A handful of points is found at once by a thread:
+// 1M queries, k = 1, 2,306 points 0.27 and 0.25, 10,000 0.29 and 0.31; k = 2,
+// 100 points 0.25 and 0.21, 300 0.26 and 0.25 (20,000 queries 0.12 and 0.13).
 __host__ __device__ inline bool group_pays(uint32_t numQueries, uint32_t numPrims, int k)
 {
   const uint64_t q = numQueries, p = numPrims;
-  if (k == 1) return q >= 4 * p && p >= 32768;
-  if (k <= 4) return q >= 2 * p && p >= 1024;
+  if (k == 1) return q >= 4 * p && p >= 8192;
+  if (k <= 4) return ((q >= 2 * p && q >= 32768) || q >= 8 * p) && p >= 256;
   if (k <= 16) return (q >= p || (2 * q >= p && q >= (1u << 19))) && p >= 32;
   return 2 * q >= p && p >= 32;
 }

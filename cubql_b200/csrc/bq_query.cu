@@ -56,13 +56,17 @@ inline bool cp_order_pays(uint32_t nq, uint32_t numNodes)
   return nq >= (3u << 16) || (nq >= (1u << 16) && (uint64_t)nq * numNodes >= 1700000000000ull);
 }
 inline uint32_t knn_order_min(int k) { return k <= 8 ? 4096 : 2; }
-// Longest lists whose searches, a thread each, do not walk in step: inserting
-// into them costs little, so leaves are better taken at once (2M points and
-// queries, plain and in step, ms: k = 1 1.01 and 1.26, 4 1.84 and 1.99, 5 2.31
-// and 2.47, 8 3.09 and 3.01, 16 6.75 and 5.08).  Leaves of several prims cost
-// more (400,000 points, leaves of eight, 2,000 queries, k = 4: 0.201 and
-// 0.177).
-constexpr int KNN_PLAIN_MAX = 5;
+// Whether searches, a thread each, walk in step.  Inserting into a short list
+// costs little, so leaves are better taken at once (2M points and queries,
+// plain and in step, ms: k = 1 1.01 and 1.26, 4 1.84 and 1.99, 5 2.31 and 2.47,
+// 8 3.09 and 3.01, 16 6.75 and 5.08), unless they hold several prims (400,000
+// points, leaves of eight, 2,000 queries, k = 4: 0.201 and 0.177) or the
+// queries are few and far between (200,000 points, 5,000 queries: k = 1 0.138
+// and 0.140, 2 equal, 4 0.199 and 0.178).
+inline bool knn_steps(int k, uint32_t nq, uint32_t numPrims, uint32_t numNodes)
+{
+  return k > 5 || numPrims / 2 >= numNodes || (k > 2 && nq < (1u << 16));
+}
 
 // rootBox: lower xyz, upper xyz (the first 24 bytes of a binary root node)
 template <bool HILBERT>
@@ -485,7 +489,7 @@ void launch_knn(const bq_bvh3f *bvh, const float *points, const float *queries, 
                qs.ovfCount);
   } else {
     ProfScope ps("query.knn", s);
-    const bool step = k > KNN_PLAIN_MAX || bvh->numPrims / 2 >= bvh->numNodes;
+    const bool step = knn_steps(k, nq, bvh->numPrims, bvh->numNodes);
     launch_pdl(step ? k_knn<K, TIE, STACK, true> : k_knn<K, TIE, STACK, (K > 8)>, dim3(div_up(nq, block)), dim3(block),
                KNN_SMEM_STACK * sizeof(StackEntry) * block, s, nodes, bvh->primIDs, points, queries, qs.order, nq, k,
                maxSqr, ids, d, nf, qs.ovfList, qs.ovfCount);

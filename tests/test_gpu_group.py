@@ -42,7 +42,7 @@ def _knn_both_ways(bq, bvh, tp, tq, k, shared, **kw):
 @pytest.mark.parametrize("k", [2, 4, 5, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("n,leaf", [(32, 1), (1024, 1), (1024, 40), (3000, 8)])
 def test_knn_shared_search_equals_one_thread_per_query(bq, extra, k, n, leaf):
-    nq = (6016 if k <= 16 else 1504) + extra
+    nq = (24064 if k <= 4 else 6016 if k <= 16 else 1504) + extra
     pts, qs = W.uniform_points(n), W.uniform_points(nq, W.SEED_QUERIES, -0.1, 1.1)
     tp, tq = _cuda(pts), _cuda(qs)
     bvh = bq.cuda.radixBuilder(_cuda(boxes_np(pts)), bq.BuildConfig(makeLeafThreshold=leaf))
@@ -53,8 +53,9 @@ def test_knn_shared_search_equals_one_thread_per_query(bq, extra, k, n, leaf):
 
 # either side of each line that decides between the shared search and a thread a query
 @pytest.mark.parametrize("n,nq,k,shared", [
-    (32768, 131072, 1, True), (32768, 131071, 1, False), (32767, 140000, 1, False),
-    (5000, 10000, 4, True), (5000, 9999, 4, False), (1023, 9999, 4, False),
+    (8192, 32768, 1, True), (8192, 32767, 1, False), (8191, 40000, 1, False),
+    (16384, 32768, 4, True), (16384, 32767, 4, False), (20000, 39999, 2, False), (1000, 8000, 3, True),
+    (1000, 7999, 3, False), (256, 5000, 2, True), (255, 5000, 4, False),
     (6000, 6000, 5, True), (6000, 5999, 16, False), (1 << 20, 1 << 19, 9, True), (1 << 20, (1 << 19) - 1, 9, False),
     (32, 5000, 16, True), (31, 5000, 16, False), (4000, 2000, 17, True), (4000, 1999, 32, False),
     (2000, 4096, 8, True), (2000, 4095, 8, False), (5000, 9000, 33, False)])
@@ -66,7 +67,7 @@ def test_knn_where_the_shared_search_begins(bq, n, nq, k, shared):
 
 
 @pytest.mark.parametrize("tie", [0, 1])
-@pytest.mark.parametrize("k", [1, 4, 5, 6])
+@pytest.mark.parametrize("k", [1, 2, 3, 5, 6])
 @pytest.mark.parametrize("leaf", [1, 8])
 def test_knn_plain_and_in_step_match_oracle(bq, oracle, tie, k, leaf):
     """A thread a query, on its own (short lists over short leaves) and with
@@ -76,9 +77,14 @@ def test_knn_plain_and_in_step_match_oracle(bq, oracle, tie, k, leaf):
     assert (bvh.numPrims // 2 >= bvh.numNodes) == (leaf == 8)
     n, pr = bvh.to_host()
     want = oracle.knn(n, pr, pts, qs, k, tie_mode=tie)
-    got = bq.points.findKNN(bvh, _cuda(pts), _cuda(qs), k, qcfg=bq.query_config(tieMode=tie))
+    cfg = bq.query_config(tieMode=tie, reorder=0)
+    got = bq.points.findKNN(bvh, _cuda(pts), _cuda(qs), k, qcfg=cfg)
     for a, b in zip(got, want):
         assert np.array_equal(a.cpu().numpy(), b)
+    many = _cuda(np.resize(qs, (65536 + 33, 3)))  # the size from which lists of three to five are plain
+    for nq in (65535, 65536, len(many)):
+        for a, b in zip(bq.points.findKNN(bvh, _cuda(pts), many[:nq], k, qcfg=cfg), got):
+            assert np.array_equal(a.cpu().numpy(), np.resize(b.cpu().numpy(), (nq,) + b.shape[1:]))
 
 
 def test_knn_shared_search_on_duplicates_and_clusters(bq):
